@@ -16,6 +16,8 @@
 
 namespace gbsb {
 
+constexpr int kHafMaxN = 32;  // matrix side cap of the hafnian and loop hafnian paths
+
 // ------------------------------------------------------------------ status
 // Per-instance status words written by the kernels (0 = ok). The host maps them
 // to the reference's value conventions (NaN for off-domain / uncertifiable).

@@ -11,11 +11,13 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "gbs_common.cuh"
 #include "gbs_kernels.cuh"
 #include "haf_dd.cuh"
 #include "haf_pt.cuh"
+#include "haf_rec.cuh"
 #include "perm_tor.cuh"
 #include "cert.cuh"
 #include "tor_lu.cuh"
@@ -123,49 +125,37 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
     r.val = acc.z;
     r.aux = acc.r;
     if (!isfinite(acc.r) || !isfinite(acc.z.re.hi) || !isfinite(acc.z.im.hi)) r.st = kStUncertified;
-  } else if (TIER == kTierCert) {
-    // same grouping as the binary64 tiers (rings of kHafRing subsets, butterfly sum
-    // per ring) so the certified value is the fp64 value bit for bit
-    const HafLayout L = haf_layout(haf_smax, true);
-    double* ring = ws + L.cring_off;
-    cball acc{mkc(0.0, 0.0), 0.0};
-    int cnt = 0;
-    for (unsigned long long k = 0; k < w.count; ++k) {
-      // each subset parks its kg balls; kHafRing lanes then run the recurrences at once
-      haf_subset_term_tc<true, REAL>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane, ring + cnt * L.cslot);
-      if (++cnt == kHafRing || k + 1 == w.count) {
-        __syncwarp();
-        acc = cb_add(acc, haf_ring_flush_cert(ring, L.cslot, cnt, n, lane, ws + L.p_off));
-        cnt = 0;
-        __syncwarp();
-      }
-    }
-    r.val = ddc_from_c(acc.z);
-    r.aux = acc.r;
-    if (!isfinite(acc.r) || !isfinite(acc.z.re) || !isfinite(acc.z.im)) r.st = kStUncertified;
   } else {
-    // the traces of kHafRing subsets are parked, then kHafRing lanes run their
-    // Newton recurrences at once (see haf_ring_flush)
-    const HafLayout L = haf_layout(haf_smax);
-    double* ring = ws + L.ring_off;
-    cplx acc = mkc(0.0, 0.0);
-    double absacc = 0.0;
-    int cnt = 0;
-    for (unsigned long long k = 0; k < w.count; ++k) {
-      haf_subset_term_tc<false, REAL>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane, ring + cnt * L.slot * 2);
-      if (++cnt == kHafRing || k + 1 == w.count) {
-        __syncwarp();
-        double ab = 0.0;
-        const cplx t = haf_ring_flush(ring, L.slot, cnt, n, lane, TIER == kTierKappa ? &ab : nullptr,
-                                      ws + L.p_off);
-        acc = cadd(acc, t);
-        absacc += ab;
-        cnt = 0;
-        __syncwarp();
+    // binary64 tiers: the recursion over pairs (haf_rec.cuh)
+    using Z = std::conditional_t<REAL, double, cplx>;
+    bool tiny = false;
+    const Z v = haf_rec_sum<Z, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+    if constexpr (REAL) r.val = ddc{dd_make(v), dd_make(0.0)};
+    else r.val = ddc_from_c(v);
+    if (TIER == kTierCert) {
+      const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+      r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj);
+      // a halving that could round absolutely refuses the certificate
+      if (__any_sync(0xffffffffu, tiny)) r.aux = INFINITY;
+      if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
+    } else if (TIER == kTierKappa) {
+      // the cancellation indicator is the sum of the moduli of the subsets' power-trace
+      // terms, so those are evaluated beside the value (haf_pt.cuh)
+      const HafLayout L = haf_layout(haf_smax);
+      double* ring = ws + L.ring_off;
+      double absacc = 0.0;
+      int cnt = 0;
+      for (unsigned long long k = 0; k < w.count; ++k) {
+        haf_subset_traces<REAL>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane, ring + cnt * L.slot * 2);
+        if (++cnt == kHafRing || k + 1 == w.count) {
+          __syncwarp();
+          absacc += haf_ring_flush(ring, L.slot, cnt, n, lane, ws + L.p_off);
+          cnt = 0;
+          __syncwarp();
+        }
       }
+      r.aux = absacc;
     }
-    r.val = ddc_from_c(acc);
-    r.aux = absacc;
   }
   return r;
 }
@@ -322,7 +312,6 @@ __device__ __forceinline__ ItemResult eval_item(const ItemLaunch& P, const InstD
 
 template <unsigned BR>
 __global__ void __launch_bounds__(256) gbs_items_kernel(ItemLaunch P) {
-  extern __shared__ __align__(128) double smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   double* ws = smem + (size_t)warp * P.ws_doubles;

@@ -1,5 +1,8 @@
-// haf_pt.cuh -- hafnian and loop hafnian by the power-trace formula, one warp per
-// subset, binary64 on the FP64 tensor cores (mma.sync .m16n8k8 / .m16n8k4 .f64).
+// haf_pt.cuh -- the subset terms of the power-trace formula for hafnians and loop
+// hafnians, one warp per subset, binary64 on the FP64 tensor cores (mma.sync .m16n8k8 /
+// .m16n8k4 .f64).  The cancellation indicator sum |term| of the kappa and auto tiers is
+// defined by these terms; the values come from the recursion over pairs (haf_rec.cuh).
+// The bound path (haf_bound_powers) also serves the certified double-double tier.
 //
 // Algorithm (the reference's, cpu_ref/hafnian.py:101-129 and
 // cpu_ref/loop_hafnian.py:65-108; device form core/hafnian.cu:41-133,
@@ -38,7 +41,6 @@
 
 namespace gbsb {
 
-constexpr int kHafMaxN = 32;                 // matrix side cap of the tensor-core path
 constexpr int kHafMaxPairs = kHafMaxN / 2;   // n
 constexpr int kHafMaxPow = (kHafMaxPairs + 1) / 2;  // h
 
@@ -66,14 +68,8 @@ struct HafLayout {
   int smax;
   int slot;  // complex entries per ring slot (smax / 2 + 1)
   int c_off, p_off, y_off, d_off, gi_off, acc_off, ring_off, total;  // in doubles
-  // certified tier only: |C|, the bound-path power, row bounds, trace-bound sums,
-  // the Newton coefficients
-  int ca_off, m_off, ym_off, bt_off, ev_off;
-  // certified tier: the ring of parked subsets' kg balls (cslot doubles per slot:
-  // entry 0 = sign, halving flag; entries 1..n = re, im, radius)
-  int cring_off, cslot;
 };
-__host__ __device__ inline HafLayout haf_layout(int smax, bool cert = false) {
+__host__ __device__ inline HafLayout haf_layout(int smax, bool /* one layout for every tier */ = false) {
   HafLayout L;
   if (smax < 2) smax = 2;
   L.smax = smax;
@@ -91,19 +87,6 @@ __host__ __device__ inline HafLayout haf_layout(int smax, bool cert = false) {
   L.ring_off = L.acc_off + 2 * np1 * 2;    // acc_p, acc_v
   L.total = L.ring_off + kHafRing * np1 * 2;
   L.total = (L.total + 1) & ~1;  // 16-byte multiple
-  L.ca_off = L.m_off = L.ym_off = L.bt_off = L.ev_off = L.cring_off = L.cslot = 0;
-  if (cert) {
-    L.ca_off = L.total;
-    L.m_off = L.ca_off + rows * cs * 2;
-    L.ym_off = L.m_off + rows * ps * 2;
-    L.bt_off = L.ym_off + rows * (h + 1);
-    L.ev_off = L.bt_off + 2 * (kHafMaxPairs + 2);
-    L.total = L.ev_off + (kHafMaxPairs + 1) * 2;
-    L.total = (L.total + 1) & ~1;
-    L.cslot = (3 * np1 + 1) & ~1;
-    L.cring_off = L.total;
-    L.total = L.cring_off + kHafRing * L.cslot;
-  }
   return L;
 }
 
@@ -739,38 +722,26 @@ __device__ __noinline__ void haf_powers_real(const double* Cr, double* P, double
   }
 }
 
-// Stage the real C = B_S X (symmetric part, rows and columns zero-padded to the
-// tiles read) and d for a real subset into the real scratch (after the layout's
-// own areas); the certified tier also gets |C| and d in the complex layout, which
-// its bound path reads.  Returns this lane's "tiny halving" flag (see the complex
-// staging in haf_subset_term_tc).
 // Entry (r, c) of the real C = B_S X as the symmetric part (x + y) / 2; zero outside
-// the s x s block and on the skipped diagonal of a plain hafnian.  `tiny` (certified
-// tier) records a halving that could round absolutely.
-template <bool CERT>
+// the s x s block and on the skipped diagonal of a plain hafnian.
 __device__ __forceinline__ double haf_real_entry(const double* __restrict__ A, int N, int s, bool loop,
-                                                 const int* gi, int r, int c, bool& tiny) {
+                                                 const int* gi, int r, int c) {
   if (r >= s || c >= s) return 0.0;
   const int rr = gi[r], cc = gi[c ^ 1];  // X swaps the columns within each pair
   if (!loop && rr == cc) return 0.0;
-  const double x = A[((size_t)rr * N + cc) * 2], y = A[((size_t)cc * N + rr) * 2];
-  if constexpr (CERT) {
-    const double w = x + y;
-    if (x != y && fabs(w) > 0.0 && fabs(w) < 4.450147717014403e-308) tiny = true;
-  }
-  return 0.5 * (x + y);
+  return 0.5 * (A[((size_t)rr * N + cc) * 2] + A[((size_t)cc * N + rr) * 2]);
 }
 
-template <bool CERT>
-__device__ __noinline__ bool haf_stage_real(const double* __restrict__ A, int N, int s, bool loop, const int* gi,
-                                            int smax, double* ws, double* rb, int lane) {
+// Stage the real C = B_S X (rows and columns zero-padded to the tiles read) and d for a
+// real subset into the real scratch (after the layout's own areas).
+static __device__ __noinline__ void haf_stage_real(const double* __restrict__ A, int N, int s, bool loop, const int* gi,
+                                            int smax, double* rb, int lane) {
   const HafRealLayout R = haf_real_layout(smax);
   double* Cr = rb + R.c_off;
   double* Dr = rb + R.d_off;
   const int rs = R.rs;
   const int rows = 16 * haf_strips(s);
   const int rcols = 8 * ((s + 7) >> 3);
-  bool tiny = false;
   const int dr = 32 / rcols, dc = 32 - dr * rcols;  // (r, c) advance per 32 elements
   int r = lane / rcols, c = lane - (lane / rcols) * rcols;
   for (int e = lane; e < rows * rcols; e += 32, r += dr, c += dc) {
@@ -778,48 +749,28 @@ __device__ __noinline__ bool haf_stage_real(const double* __restrict__ A, int N,
       c -= rcols;
       ++r;
     }
-    Cr[r * rs + c] = haf_real_entry<CERT>(A, N, s, loop, gi, r, c, tiny);
+    Cr[r * rs + c] = haf_real_entry(A, N, s, loop, gi, r, c);
   }
   if (loop)
     for (int k = lane; k < rs; k += 32) Dr[k] = k < s ? A[((size_t)gi[k] * N + gi[k]) * 2] : 0.0;
-  if constexpr (CERT) {
-    const int cs = haf_c_stride(s);
-    const int ccols = (((2 * s + 7) >> 3) << 2);
-    double* Ca = ws + haf_layout(smax, true).ca_off;
-    const int dr2 = 32 / ccols, dc2 = 32 - dr2 * ccols;
-    int r2 = lane / ccols, c2 = lane - (lane / ccols) * ccols;
-    for (int e = lane; e < rows * ccols; e += 32, r2 += dr2, c2 += dc2) {
-      if (c2 >= ccols) {
-        c2 -= ccols;
-        ++r2;
-      }
-      st_c(Ca + (r2 * cs + c2) * 2, mkc(fabs(haf_real_entry<CERT>(A, N, s, loop, gi, r2, c2, tiny)), 0.0));
-    }
-    if (loop && lane < s)
-      st_c(ws + haf_layout(smax, true).d_off + lane * 2, mkc(A[((size_t)gi[lane] * N + gi[lane]) * 2], 0.0));
-  }
-  return tiny;
 }
 
 // ---------------------------------------------------------------------------
-// Evaluate the signed power-trace term of one subset `mask` of instance A (N x N
-// complex, row-major, N = 2n even).  Returns the same ball in every lane (radius 0
-// unless CERT).  `loop` selects the loop hafnian; `ws` is this warp's workspace.
-// Binary64 tiers (CERT false): kg[1..n] and the sign are parked in the ring slot
-// `slot` (required) instead of running the Newton recurrence (haf_ring_flush runs
-// it for a whole ring); the certified tier runs it in ball arithmetic here.
-template <bool CERT, bool REAL = false>
-static __device__ cball haf_subset_term_tc(const double* __restrict__ A, int N, int n, uint32_t mask,
-                                           bool loop, double* ws, const HafLayout& Lw, int lane,
-                                           double* slot = nullptr) {
+// Traces of one subset `mask` of instance A (N x N complex, row-major, N = 2n even):
+// kg[1..n] and the sign are parked in the ring slot `slot`; haf_ring_flush turns a
+// whole ring of them into the moduli of the subsets' terms.  `loop` selects the loop
+// hafnian; `ws` is this warp's workspace.
+template <bool REAL>
+static __device__ void haf_subset_traces(const double* __restrict__ A, int N, int n, uint32_t mask, bool loop,
+                                         double* ws, const HafLayout& Lw, int lane, double* slot) {
   const int m = __popc(mask);
   if (m == 0) {
-    if (slot && lane == 0) st_c(slot, mkc(0.0, 0.0));  // empty subset: term 0 (n >= 1)
-    return cball{mkc(n == 0 ? 1.0 : 0.0, 0.0), 0.0};
+    if (lane == 0) st_c(slot, mkc(0.0, 0.0));  // empty subset: term 0 (n >= 1)
+    return;
   }
   const int s = 2 * m;
   const int cs = haf_c_stride(s), ps = haf_p_stride(s, Lw.smax > 16);
-  const int h = (n + 1) / 2, hp1 = h + 1;
+  const int h = (n + 1) / 2;
   const int rows = 16 * haf_strips(s);
   double* Cs = ws + Lw.c_off;
   double* P = ws + Lw.p_off;        // one strip of the power
@@ -828,11 +779,6 @@ static __device__ cball haf_subset_term_tc(const double* __restrict__ A, int N, 
   int* gi = reinterpret_cast<int*>(ws + Lw.gi_off);
   double* acc_p = ws + Lw.acc_off;  // p[0..n]
   double* acc_v = acc_p + Lw.slot * 2;
-  double* Ca = ws + Lw.ca_off;
-  double* M = ws + Lw.m_off;
-  double* Ym = ws + Lw.ym_off;
-  double* bT = ws + Lw.bt_off;                  // trace bound sums T[k]
-  double* bV = bT + (kHafMaxPairs + 2);         // loop bound sums V[k]
 
   // ---- stage C = B_S X (rows padded to 16 per strip with zeros) and d
   if (lane < s) {
@@ -841,91 +787,48 @@ static __device__ cball haf_subset_term_tc(const double* __restrict__ A, int N, 
     gi[lane] = 2 * (__ffs(mm) - 1) + (lane & 1);
   }
   __syncwarp();
-  bool tiny_halving = false;  // certified tier: see the staging below
   if constexpr (REAL) {
-    tiny_halving = haf_stage_real<CERT>(A, N, s, loop, gi, Lw.smax, ws, ws + Lw.total, lane);
+    haf_stage_real(A, N, s, loop, gi, Lw.smax, ws + Lw.total, lane);
   } else {
     const int ccols = (((2 * s + 7) >> 3) << 2);  // columns read by the n-tiles (>= s)
     // rows s..rows-1 stay zero: they are the padding rows of the power-2 A operand
     const int dr = 32 / ccols, dc = 32 - dr * ccols;  // (r, c) advance per 32 elements
     int r = lane / ccols, c = lane - (lane / ccols) * ccols;
-    if constexpr (!CERT) {
-      // without divergent branches: rows < s element by element (a padding column
-      // loads a valid entry and stores zero), then the padding rows as zeros over the
-      // whole row stride.  The symmetric part (A + A^T)/2 is staged: see below.
-      for (int e = lane; e < s * ccols; e += 32, r += dr, c += dc) {
-        const bool wrap = c >= ccols;
-        c = wrap ? c - ccols : c;
-        r = wrap ? r + 1 : r;
-        const bool in = c < s;
-        const int rr = gi[r], cc = gi[in ? (c ^ 1) : 0];  // X swaps the columns within each pair
-        const cplx x = ld_c(A + ((size_t)rr * N + cc) * 2), y = ld_c(A + ((size_t)cc * N + rr) * 2);
-        const cplx v = cscale(cadd(x, y), 0.5);
-        st_c(Cs + (r * cs + c) * 2, (in && (loop || rr != cc)) ? v : mkc(0.0, 0.0));
-      }
-      for (int e = lane; e < (rows - s) * cs; e += 32) st_c(Cs + (s * cs + e) * 2, mkc(0.0, 0.0));
-    } else
-    for (int e = lane; e < rows * ccols; e += 32, r += dr, c += dc) {
-      if (c >= ccols) {
-        c -= ccols;
-        ++r;
-      }
-      cplx v = mkc(0.0, 0.0);
-      if (c < s && r < s) {
-        const int rr = gi[r], cc = gi[c ^ 1];  // X swaps the columns within each pair
-        if (loop || rr != cc) {
-          // the symmetric part (A + A^T)/2, exact for a symmetric A: the half-power
-          // identities need B_S symmetric, and the reference's n-1 products of the
-          // raw entries agree with those of the symmetric part to second order in
-          // the antisymmetric part
-          const cplx x = ld_c(A + ((size_t)rr * N + cc) * 2), y = ld_c(A + ((size_t)cc * N + rr) * 2);
-          v = cscale(cadd(x, y), 0.5);
-          if constexpr (CERT) {
-            // halving a sum below twice the smallest normal can round absolutely: no
-            // certificate for such an entry (the relative input bound would not hold)
-            const cplx w = cadd(x, y);
-            if ((x.re != y.re || x.im != y.im) && fmin(fabs(w.re) > 0.0 ? fabs(w.re) : 1.0,
-                                                       fabs(w.im) > 0.0 ? fabs(w.im) : 1.0) < 4.450147717014403e-308)
-              tiny_halving = true;
-          }
-        }
-      }
-      st_c(Cs + (r * cs + c) * 2, v);
-      if constexpr (CERT) st_c(Ca + (r * cs + c) * 2, mkc(ru_abs_c(v), 0.0));
+    // without divergent branches: rows < s element by element (a padding column
+    // loads a valid entry and stores zero), then the padding rows as zeros over the
+    // whole row stride.  The symmetric part (A + A^T)/2 is staged: the half-power
+    // identities need B_S symmetric, and the n-1 products of the raw entries agree with
+    // those of the symmetric part to second order in the antisymmetric part.
+    for (int e = lane; e < s * ccols; e += 32, r += dr, c += dc) {
+      const bool wrap = c >= ccols;
+      c = wrap ? c - ccols : c;
+      r = wrap ? r + 1 : r;
+      const bool in = c < s;
+      const int rr = gi[r], cc = gi[in ? (c ^ 1) : 0];  // X swaps the columns within each pair
+      const cplx x = ld_c(A + ((size_t)rr * N + cc) * 2), y = ld_c(A + ((size_t)cc * N + rr) * 2);
+      const cplx v = cscale(cadd(x, y), 0.5);
+      st_c(Cs + (r * cs + c) * 2, (in && (loop || rr != cc)) ? v : mkc(0.0, 0.0));
     }
+    for (int e = lane; e < (rows - s) * cs; e += 32) st_c(Cs + (s * cs + e) * 2, mkc(0.0, 0.0));
     if (loop && lane < s) st_c(Dv + lane * 2, ld_c(A + ((size_t)gi[lane] * N + gi[lane]) * 2));
     else if (loop && lane < ((s + 3) & ~3)) st_c(Dv + lane * 2, mkc(0.0, 0.0));  // whole column tiles
   }
   for (int k = lane; k <= n; k += 32) {
     st_c(acc_p + 2 * k, mkc(0.0, 0.0));
     st_c(acc_v + 2 * k, mkc(0.0, 0.0));
-    if constexpr (CERT) { bT[k] = 0.0; bV[k] = 0.0; }
   }
   __syncwarp();
-  if constexpr (CERT) {
-    if (loop && lane < rows) Ym[lane * hp1] = lane < s ? ru_abs_c(ld_c(Dv + lane * 2)) : 0.0;
-  }
   // p_1 = tr(C)
   if constexpr (REAL) {
     const HafRealLayout R = haf_real_layout(Lw.smax);
     const double* Cr = ws + Lw.total + R.c_off;
-    const double d = lane < s ? Cr[lane * R.rs + lane] : 0.0;
-    const double t = warp_sum_d(d);
+    const double t = warp_sum_d(lane < s ? Cr[lane * R.rs + lane] : 0.0);
     if (lane == 0) st_c(acc_p + 2, mkc(t, 0.0));
-    if constexpr (CERT) {
-      const double a1 = warp_sum_ru(fabs(d));
-      if (lane == 0) bT[1] = a1;
-    }
   } else {
     cplx t = mkc(0.0, 0.0);
     if (lane < s) t = ld_c(Cs + (lane * cs + lane) * 2);
     t = warp_sum_c(t);
     if (lane == 0) st_c(acc_p + 2, t);
-    if constexpr (CERT) {
-      double a1 = lane < s ? ru_abs_c(ld_c(Cs + (lane * cs + lane) * 2)) : 0.0;
-      a1 = warp_sum_ru(a1);
-      if (lane == 0) bT[1] = a1;
-    }
   }
   __syncwarp();
 
@@ -951,160 +854,29 @@ static __device__ cball haf_subset_term_tc(const double* __restrict__ A, int N, 
     if (Lw.smax <= 16) haf_powers<4>(Cs, P, Y, Dv, acc_p, acc_v, s, cs, ps, n, h, loop, lane);
     else haf_powers<8>(Cs, P, Y, Dv, acc_p, acc_v, s, cs, ps, n, h, loop, lane);
   }
-  if constexpr (CERT) {
-    __syncwarp();
-    if (s <= 16) haf_bound_powers<4, 1>(Ca, M, Ym, Dv, bT, s, cs, ps, n, h, loop, lane);
-    else haf_bound_powers<8, 2>(Ca, M, Ym, Dv, bT, s, cs, ps, n, h, loop, lane);
+  __syncwarp();
+  // ---- kg_k parked by lane k
+  if (lane == 0) st_c(slot, mkc(((n - m) & 1) ? -1.0 : 1.0, 0.0));
+  if (lane >= 1 && lane <= n) {
+    const int k = lane;
+    cplx g = cscale(ld_c(acc_p + 2 * k), 0.5);
+    if (loop) g = cadd(g, cscale(ld_c(acc_v + 2 * k), (double)k));
+    st_c(slot + 2 * k, g);
   }
   __syncwarp();
-
-  if constexpr (CERT) {
-    // loop bound sums V[k] = sum_i Ym[i^1][a] Ym[i][b] (the values v_k came with the powers)
-    if (loop) {
-      for (int k = 1; k <= n; ++k) {
-        const int aa = (k - 1) >> 1, bb = k - 1 - aa;
-        double vb = lane < s ? ru_mul(Ym[(lane ^ 1) * hp1 + aa], Ym[lane * hp1 + bb]) : 0.0;
-        vb = warp_sum_ru(vb);
-        if (lane == 0) bV[k] = vb;
-      }
-      __syncwarp();
-    }
-  }
-
-  // ---- Newton recurrence (certified: lane 0, then broadcast through shared memory;
-  // binary64 tiers: kg_k parked by lane k, the recurrence runs in haf_ring_flush)
-  bool tiny_any = false;  // certified tier: a halving anywhere refuses the certificate
-  if constexpr (CERT) tiny_any = __any_sync(0xffffffffu, tiny_halving);
-  if (!CERT || lane == 0) {
-    if constexpr (CERT) {
-      // value-path coefficients: E_a <= c_a M_a with M_a = |C|^a, M_a <= phi_a M^_a
-      const double g2s = gamma_ru((double)(2 * s), 2.0 * kU);  // FP64 MMA, faithful rounding
-      const double sq2 = 1.4142135623730952;
-      const double g64 = ru_mul(sq2, gamma_ru(64.0, kU));
-      const double gy = ru_mul(sq2, gamma_ru((double)(s + 4), kU));
-      // loop term: complex products (4u) summed sequentially over the rows of each
-      // strip, then the strips (at most s + 1 sums; sqrt(2) gamma_{s+4} <= gamma_{2s+8}
-      // per component pair)
-      const double gv = ru_add(4.0 * kU, gamma_ru(2.0 * s + 8.0, kU));
-      // Input error: the staged C^ is the rounded symmetric part, |C - C^| <= c1 |C^|
-      // with c1 = u/(1-u) (exactly 0 for a symmetric A; charged regardless), so
-      // |C^a| <= t_a M_a with t_a = (1 + c1)^a, and the power errors E_a <= c_a M_a
-      // follow c_1 = c1, c_{a+1} = c_a + c1 t_a + sqrt2 gamma_2s (t_a + c_a).
-      const double c1 = kUc;
-      double ca[kHafMaxPow + 2], ph[kHafMaxPow + 2], ka[kHafMaxPow + 2], ta[kHafMaxPow + 2];
-      ca[0] = 0.0; ph[0] = 1.0; ca[1] = c1; ph[1] = 1.0; ta[0] = 1.0; ta[1] = ru_add(1.0, c1);
-      for (int a = 1; a <= h; ++a) {
-        ca[a + 1] = ru_add(ru_add(ca[a], ru_mul(c1, ta[a])), ru_mul(ru_mul(sq2, g2s), ru_add(ta[a], ca[a])));
-        ph[a + 1] = ru_div(ph[a], rd_sub(1.0, g2s));
-        ta[a + 1] = ru_mul(ta[a], ru_add(1.0, c1));
-      }
-      ka[0] = 0.0;
-      for (int a = 1; a <= h; ++a) ka[a] = ru_add(ca[a], ru_mul(gy, ru_add(ta[a], ca[a])));
-      cball kgb[kHafMaxPairs + 1];
-      for (int k = 1; k <= n; ++k) {
-        double ep;
-        if (k == 1) {
-          ep = ru_mul(ru_add(gamma_ru(6.0, kU), c1), bT[1]);
-        } else if ((k & 1) == 0) {
-          const int a = k / 2;
-          double f = ru_add(ru_mul(ca[a], ru_add(ru_mul(2.0, ta[a]), ca[a])),
-                            ru_mul(g64, ru_mul(ru_add(ta[a], ca[a]), ru_add(ta[a], ca[a]))));
-          ep = ru_mul(ru_mul(f, ru_mul(ph[a], ph[a])), bT[k]);
-        } else {
-          const int a = (k + 1) / 2;
-          double f = ru_add(ru_add(ru_add(ru_mul(ca[a], ta[a - 1]), ru_mul(ca[a - 1], ta[a])),
-                                   ru_mul(ca[a], ca[a - 1])),
-                            ru_mul(g64, ru_mul(ru_add(ta[a], ca[a]), ru_add(ta[a - 1], ca[a - 1]))));
-          ep = ru_mul(ru_mul(f, ru_mul(ph[a], ph[a - 1])), bT[k]);
-        }
-        cball g{cscale(ld_c(acc_p + 2 * k), 0.5), ru_mul(0.5, ep)};
-        if (loop) {
-          const int aa = (k - 1) >> 1, bb = k - 1 - aa;
-          double f = ru_add(ru_add(ru_add(ru_mul(ka[aa], ta[bb]), ru_mul(ka[bb], ta[aa])), ru_mul(ka[aa], ka[bb])),
-                            ru_mul(gv, ru_mul(ru_add(ta[aa], ka[aa]), ru_add(ta[bb], ka[bb]))));
-          double evb = ru_mul(0.5, ru_mul(ru_mul(f, ru_mul(ph[aa], ph[bb])), bV[k]));
-          g = cb_add(g, cb_scale(cball{ld_c(acc_v + 2 * k), evb}, (double)k));
-        }
-        kgb[k] = g;
-      }
-      // parked for the recurrence (haf_ring_flush_cert: one lane per subset)
-      slot[0] = ((n - m) & 1) ? -1.0 : 1.0;
-      slot[1] = tiny_any ? 1.0 : 0.0;
-      for (int k = 1; k <= n; ++k) {
-        slot[3 * k] = kgb[k].z.re;
-        slot[3 * k + 1] = kgb[k].z.im;
-        slot[3 * k + 2] = kgb[k].r;
-      }
-    } else {
-      if (lane == 0) st_c(slot, mkc(((n - m) & 1) ? -1.0 : 1.0, 0.0));
-      if (lane >= 1 && lane <= n) {
-        const int k = lane;
-        cplx g = cscale(ld_c(acc_p + 2 * k), 0.5);
-        if (loop) g = cadd(g, cscale(ld_c(acc_v + 2 * k), (double)k));
-        st_c(slot + 2 * k, g);
-      }
-    }
-  }
-  __syncwarp();
-  if constexpr (!CERT) {
-    return cball{mkc(0.0, 0.0), 0.0};
-  } else {
-    return cball{mkc(0.0, 0.0), 0.0};  // the term comes from haf_ring_flush_cert
-  }
 }
 
-// Certified tier: the Newton recurrences of `cnt` parked subsets in ball arithmetic,
-// one lane each -- the operations of the one-subset recurrence, in its order, with
-// e_j interleaved in the idle power buffer `e` (3 doubles per ball) -- and the ball
-// sum of their signed terms over the lanes (warp_sum_cb, the grouping of the
-// binary64 ring, so the value is the fp64 value bit for bit).  A subset with a
-// halving that could round absolutely gets an infinite radius.
-__device__ __forceinline__ cball haf_ring_flush_cert(const double* ring, int slotw, int cnt, int n, int lane,
-                                                     double* e) {
-  cball b{mkc(0.0, 0.0), 0.0};
-  if (lane < cnt) {
-    const double* sl = ring + lane * slotw;
-    const double sign = sl[0];
-    if (sign != 0.0) {
-      double* el = e + lane * 3;
-      constexpr int es = kHafRing * 3;  // doubles between e_j and e_{j+1} of a lane
-      el[0] = 1.0;
-      el[1] = 0.0;
-      el[2] = 0.0;
-      for (int j = 1; j <= n; ++j) {
-        cball acc{mkc(0.0, 0.0), 0.0};
-        for (int k = 1; k <= j; ++k) {
-          const double* ek = el + (j - k) * es;
-          acc = cb_add(acc, cb_mul(cball{mkc(sl[3 * k], sl[3 * k + 1]), sl[3 * k + 2]}, cball{mkc(ek[0], ek[1]), ek[2]}));
-        }
-        const cball ej = cb_div_int(acc, (double)j);
-        double* ed = el + j * es;
-        ed[0] = ej.z.re;
-        ed[1] = ej.z.im;
-        ed[2] = ej.r;
-      }
-      const double* en = el + n * es;
-      const cplx coeff = mkc(en[0], en[1]);
-      b = cball{sign < 0.0 ? cneg(coeff) : coeff, sl[1] != 0.0 ? INFINITY : en[2]};
-    }
-  }
-  return warp_sum_cb(b);
-}
-
-// Run the Newton recurrence of `cnt` parked subsets, one lane each, and return
-// the sum of their signed terms (every lane gets it; fixed butterfly order) and,
-// in *absacc, the sum of |term|.  The coefficients e_0..e_n of lane l live in
-// shared memory at e + (j kHafRing + l) complex entries (`e`: (n + 1) kHafRing
-// complex entries that are free while the ring is flushed, the power buffer): a
-// per-thread array would sit in local memory, whose stacks (8.7 KB per warp)
-// overflow the L1 left beside the shared-memory workspaces.
-__device__ __forceinline__ cplx haf_ring_flush(const double* ring, int slotw, int cnt, int n, int lane,
-                                               double* absacc, double* e) {
+// Run the Newton recurrence of `cnt` parked subsets, one lane each, and return the sum
+// of the moduli of their terms (every lane gets it; fixed butterfly order).  The
+// coefficients e_0..e_n of lane l live in shared memory at e + (j kHafRing + l) complex
+// entries (`e`: (n + 1) kHafRing complex entries that are free while the ring is
+// flushed, the power buffer): a per-thread array would sit in local memory, whose
+// stacks (8.7 KB per warp) overflow the L1 left beside the shared-memory workspaces.
+__device__ __forceinline__ double haf_ring_flush(const double* ring, int slotw, int cnt, int n, int lane, double* e) {
   cplx term = mkc(0.0, 0.0);
   if (lane < cnt) {
     const double* sl = ring + lane * slotw * 2;
-    const double sign = sl[0];
-    if (sign != 0.0) {
+    if (sl[0] != 0.0) {
       double* el = e + lane * 2;
       constexpr int es = kHafRing * 2;  // doubles between e_j and e_{j+1} of a lane
       st_c(el, mkc(1.0, 0.0));
@@ -1113,11 +885,10 @@ __device__ __forceinline__ cplx haf_ring_flush(const double* ring, int slotw, in
         for (int k = 1; k <= j; ++k) acc = cadd(acc, cmul(ld_c(sl + 2 * k), ld_c(el + (j - k) * es)));
         st_c(el + j * es, mkc(acc.re / j, acc.im / j));
       }
-      term = cscale(ld_c(el + n * es), sign);
+      term = ld_c(el + n * es);
     }
   }
-  if (absacc) *absacc = warp_sum_d(cabs_fast(term));
-  return warp_sum_c(term);
+  return warp_sum_d(cabs_fast(term));
 }
 
 }  // namespace gbsb

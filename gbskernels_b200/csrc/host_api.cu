@@ -29,6 +29,7 @@
 #include "gbs_kernels.cuh"
 #include "haf_dd.cuh"
 #include "haf_pt.cuh"
+#include "haf_rec.cuh"
 #include "tor_lu.cuh"
 #include "tor_warp.cuh"
 #include "tor_warp_dd.cuh"
@@ -91,6 +92,7 @@ constexpr int kPermCap = 28;
 constexpr int kHafCap = kHafMaxN;   // 32 (after odd-N loop augmentation)
 constexpr int kTorCapModes = 24;        // batched torontonian
 constexpr int kTorSingleCapModes = 32;  // single-large torontonian (binary64 tiers)
+constexpr size_t kMaxBlockSmem = 227 * 1024;  // shared memory of one block
 
 // ------------------------------------------------------------------ requests and plans
 struct Req {
@@ -180,7 +182,7 @@ static double item_cost(int fn, int dim, unsigned long long count, int tier, int
         c = (double)count * dim * dim * dim;
         break;
       }
-      const int qd = n - std::min(n, 4);
+      const int qd = n - std::min(n, kTorTailDD);
       c = (tier == kTierDD || tier == kTierCertDD) ? 20.0 * (double)count * std::ldexp(1.0, qd - param) * 16.0 * (36.0 * qd + 900.0)
                           : (double)count * std::ldexp(1.0, q - param) * 32.0 * (36.0 * q + 1400.0);
       break;
@@ -262,6 +264,20 @@ static int plan_instance(Plan& P, int fn, int tier, int dim_eval, bool real_in, 
   return idx;
 }
 
+// haf_rec_ws from a table (computed once; a plan asks for every instance).
+static int rec_ws(int n, bool loop, bool real) {
+  struct Table {
+    int w[kHafMaxN / 2 + 1][2][2];
+    Table() {
+      for (int i = 0; i <= kHafMaxN / 2; ++i)
+        for (int l = 0; l < 2; ++l)
+          for (int r = 0; r < 2; ++r) w[i][l][r] = haf_rec_ws(i, l != 0, r != 0);
+    }
+  };
+  static const Table t;
+  return t.w[n][loop ? 1 : 0][real ? 1 : 0];
+}
+
 static int ws_for_plan(const Plan& P) {
   int ws = 2;
   for (const InstDesc& d : P.insts) {
@@ -272,8 +288,11 @@ static int ws_for_plan(const Plan& P) {
     else if (fn == kFnTor && (tier == kTierDD || tier == kTierCertDD)) w = tor_d_layout(d.dim / 2, tier == kTierCertDD).total;
     else if (fn == kFnTor) w = tor_w_layout(d.dim / 2, tier == kTierCert).total;
     else if (tier == kTierDD || tier == kTierCertDD) w = haf_dd_layout(P.haf_smax, tier == kTierCertDD).total;
-    else if (d.real_in) w = haf_layout(P.haf_smax, tier == kTierCert).total + haf_real_layout(P.haf_smax).total;
-    else w = haf_layout(P.haf_smax, tier == kTierCert).total;
+    else {
+      w = rec_ws(d.dim / 2, fn == kFnLhaf, d.real_in);
+      if (tier == kTierKappa)  // the power-trace terms use a workspace of the launch's largest side
+        w = std::max(w, haf_layout(P.haf_smax).total + (d.real_in ? haf_real_layout(P.haf_smax).total : 0));
+    }
     ws = std::max(ws, w);
   }
   return (ws + 3) & ~3;  // 32-byte multiple per warp
@@ -368,7 +387,7 @@ static cudaError_t grow_pin(PinBuf& b, size_t bytes) {
 // Validate + normalise one request.  Returns 0 or an error code; on success fills
 // the evaluated side length (odd loop hafnian augmented) and the real-input flag.
 // A hafnian or loop hafnian given as host data with every imaginary part zero runs
-// the real power loop in the binary64 tiers (fp64, indicator, certified; the
+// in real arithmetic in the binary64 tiers (fp64, indicator, certified; the
 // double-double walks are complex only).  Resident-state requests stay complex.
 static bool haf_real_path(const Req& r) {
   if (r.state || !r.mat) return false;
@@ -675,7 +694,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     if (smem_per_warp >= 8192) {
       int best = 0;
       for (int w = 1; w <= 4; w <<= 1) {
-        if ((size_t)w * smem_per_warp > 200 * 1024) break;
+        if ((size_t)w * smem_per_warp > kMaxBlockSmem) break;
         const int resident = occ_any(G.br, L, w) * w;
         if (resident > best) { best = resident; warps = w; }
       }
@@ -685,7 +704,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
       const int tw = tuned_warps(ft_fn(P.insts[0].ft), ft_tier(P.insts[0].ft), P.insts[0].dim);
       if (tw > 0) warps = tw;
     }
-    while (warps > 1 && (size_t)warps * smem_per_warp > 200 * 1024) warps >>= 1;
+    while (warps > 1 && (size_t)warps * smem_per_warp > kMaxBlockSmem) warps >>= 1;
     const int bps = occ_any(G.br, L, warps);
     if (bps <= 0) return fail(cudaErrorInvalidConfiguration, "work item kernel does not fit on an SM");
     const long long want_blocks = (nit + warps - 1) / warps;

@@ -18,8 +18,8 @@
 // can be read by the GPU later.
 //
 // The result equals gbs_haf_host's bit for bit for complex input (same work items,
-// same kernel).  Every input here takes the complex power loop; gbs_haf_host runs
-// a real input (every imaginary part zero) through the real loop, so for real
+// same kernel).  Every input here takes the complex recursion; gbs_haf_host runs
+// a real input (every imaginary part zero) through the real one, so for real
 // input the two agree to rounding.
 #include <cuda_runtime.h>
 
@@ -193,7 +193,7 @@ int gbs_haf_noalloc(const double* d_mats, int N, int batch, double* d_out, void*
   L.aux_out = d_aux;
   L.st_out = d_st;
   L.haf_smax = N;
-  L.ws_doubles = (haf_layout(N).total + 3) & ~3;
+  L.ws_doubles = haf_rec_ws(n, false, false);
   constexpr unsigned BR = br1(kFnHaf, kTierFp64);
   const int bps = occ_br<BR>(L, 1);
   int dev = 0, sms = 0;

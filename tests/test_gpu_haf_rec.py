@@ -1,0 +1,59 @@
+"""The hafnian recursion (csrc/haf_rec.cuh) at the sizes and splits where its walk changes:
+no prefix, a prefix, the depth-first part (blocks of 6 and 7 pairs), several blocks per
+item, single-subset items; real and complex, hafnian and loop hafnian, against the
+binary128 oracle; the indicator and certified tiers give the same value."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _mat(N, real, seed):
+    g = np.random.default_rng(seed)
+    X = g.standard_normal((N, N)) + (0 if real else 1j * g.standard_normal((N, N)))
+    return ((X + X.T) / 4).astype(np.complex128)
+
+
+@pytest.mark.parametrize("N", [1, 2, 4, 9, 10, 12, 14, 15, 16, 18])
+def test_every_split_vs_oracle(gpu, lib, orc, N):
+    n = (N + 1) // 2
+    for func, code in (("haf", 1), ("lhaf", 2)):
+        if func == "haf" and N % 2:
+            continue
+        for real in (False, True):
+            A = _mat(N, real, 100 + N)
+            t, absn = getattr(orc, func)(A, "quad", with_absnorm=True)
+            # the recursion's terms are smaller than the power trace's (absn): a few n u of it
+            tol = 32 * n * U * absn
+            f = getattr(gpu, f"{func}_batched")
+            for split in sorted({0, 1, 4, 5, 6, 7, 8, n} | {-1}):
+                if split > n:
+                    continue
+                assert lib.gbs_set_split(code, 0, 2 * n, split, 0) == 0
+                try:
+                    v = f(A[None])[0]
+                    vc, dc = f(A[None], precision="certified", return_diagnostics=True)
+                    _, dk = f(A[None], precision="auto", return_diagnostics=True)
+                finally:
+                    lib.gbs_set_split(code, 0, 2 * n, -1, 0)
+                assert abs(v - t) <= tol, (func, real, split, v, t)
+                assert vc[0] == v and abs(v - t) <= dc[0]["abs_error_bound"] + U * abs(t), (func, real, split)
+                assert dk[0]["cancellation"] == pytest.approx(absn / abs(t), rel=1e-6), (func, real, split)
+
+
+@pytest.mark.parametrize("N", [30, 32])
+def test_largest_sizes_factorise(gpu, N):
+    """A direct sum: the hafnians of the blocks multiply (complex and real)."""
+    for real in (False, True):
+        A, B = _mat(14, real, 1), _mat(N - 14, real, 2)
+        blk = np.zeros((N, N), complex)
+        blk[:14, :14], blk[14:, 14:] = A, B
+        p = np.random.default_rng(3).permutation(N)
+        for f in ("haf", "lhaf"):
+            v, d = getattr(gpu, f)(blk[np.ix_(p, p)], precision="certified", return_diagnostics=True)
+            want = getattr(gpu, f)(A) * getattr(gpu, f)(B)
+            assert abs(v - want) <= d["abs_error_bound"] + 1e-9 * abs(want), (f, real, v, want)
