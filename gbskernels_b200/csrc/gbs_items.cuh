@@ -21,6 +21,7 @@
 #include "perm_tor.cuh"
 #include "cert.cuh"
 #include "tor_lu.cuh"
+#include "tor_rec.cuh"
 #include "tor_warp.cuh"
 #include "tor_warp_dd.cuh"
 
@@ -165,7 +166,6 @@ __device__ ItemResult tor_item(const double* __restrict__ mats, const InstDesc& 
                                double* ws, int lane) {
   ItemResult r{ddc{dd_make(0.0), dd_make(0.0)}, 0.0, kStOk};
   const int n = d.dim / 2;
-  const int dim = d.dim;
   const double* Oc = mats + d.off;
   if (!d.real_in) {
     // complex O (binary64 tiers only; the host refuses the others): one warp per
@@ -192,80 +192,50 @@ __device__ ItemResult tor_item(const double* __restrict__ mats, const InstDesc& 
     }
     return r;
   }
-  if constexpr (TIER != kTierDD && TIER != kTierCertDD) {
-    // binary64 tiers: warp-cooperative prefix walk with the 32-subset register tail
-    // (tor_warp.cuh); one work item = w.count prefix patterns over the first d.param
-    // prefix modes, walked one after another by the whole warp
-    const TorWLayout Lw = tor_w_layout(n, TIER == kTierCert);
-    double* rho = ws + Lw.rho_off;
-    bool proved = true;
-    if (TIER == kTierCert) {
-      double dmin2 = 0.0;
-      const double sigma = tor_cert_sigma(Oc, n, ws + Lw.col_off, lane, dmin2);
-      proved = sigma > 0.0;
-      tor_cert_rho(sigma, dmin2, n, rho, lane);
-    }
-    double val = 0.0, aux = 0.0;
-    bool ok = true;
-    if (proved) {
-      for (unsigned long long p = 0; p < w.count; ++p) {
-        double t = 0.0, a = 0.0;
-        ok = tor_warp_item<TIER == kTierKappa, TIER == kTierCert>(Oc, n, d.param, (uint32_t)(w.lo + p), ws, Lw,
-                                                                   rho, lane, t, a) && ok;
-        if (p == 0) {
-          val = t;
-          aux = a;
-        } else if (TIER == kTierCert) {
-          val += t;
-          aux = ru_add(ru_add(aux, a), ru_mul(kUc, fabs(val)));
-        } else {
-          val += t;
-          aux += a;
-        }
-      }
-    }
-    r.val = ddc{dd_make(val), dd_make(0.0)};
-    r.aux = aux;
-    if (!proved || !ok) r.st = TIER == kTierCert ? kStUncertified : kStOffDomain;
-    __syncwarp();
-    return r;
-  } else {
-    // double-double tiers: the same walk in double-word arithmetic with a 16-subset
-    // tail (tor_warp_dd.cuh); one work item = w.count prefix patterns.  The certified
-    // tier adds the radius (same value bit for bit).
-    constexpr bool CERT = TIER == kTierCertDD;
-    const TorDLayout Lw = tor_d_layout(n, CERT);
-    double* rho = ws + Lw.rho_off;
-    bool proved = true;
-    if (CERT) {
-      double dmin2 = 0.0;
-      const double sigma = tor_cert_sigma(Oc, n, ws + Lw.col_off, lane, dmin2);
-      proved = sigma > 0.0;
-      tor_cert_rho_dd(sigma, dmin2, n, rho, lane);
-    }
-    dd val = dd_make(0.0);
-    double aux = 0.0;
-    bool ok = true;
-    if (proved) {
-      for (unsigned long long p = 0; p < w.count; ++p) {
-        dd t = dd_make(0.0);
-        double a = 0.0;
-        ok = tor_dd_item<CERT>(Oc, n, d.param, (uint32_t)(w.lo + p), ws, Lw, rho, lane, t, a) && ok;
-        if (p == 0) {
-          val = t;
-          aux = a;
-        } else {
-          val = dd_add(val, t);
-          if (CERT) aux = ru_add(ru_add(aux, a), ru_add(ru_mul(4.0 * kU * kU, fabs(val.hi)), kUfl));
-        }
-      }
-    }
-    r.val = ddc{val, dd_make(0.0)};
-    r.aux = aux;
-    if (!proved || !ok) r.st = CERT ? kStUncertified : kStOffDomain;
-    __syncwarp();
-    return r;
+  // real O: the recursion over modes on Schur complements (tor_rec.cuh); one work item =
+  // w.count patterns over the first d.param modes.  The certified tiers' value is that of
+  // the plain tier bit for bit.
+  using S = std::conditional_t<TIER == kTierDD || TIER == kTierCertDD, dd, double>;
+  constexpr bool CERT = TIER == kTierCert || TIER == kTierCertDD;
+  constexpr int AUX = CERT ? 2 : (TIER == kTierKappa ? 1 : 0);
+  const int f = tor_rec_free(n, d.param);
+  const TorRecLayout R = tor_rec_layout(n, f, TorRec<S>::kTail, CERT, TorRec<S>::W);
+  double* rho = ws + R.rho * TorRec<S>::W;
+  bool proved = true;
+  if (CERT) {
+    double dmin2 = 0.0;
+    const double sigma = tor_cert_sigma(Oc, n, ws, lane, dmin2);
+    proved = sigma > 0.0;
+    if constexpr (TIER == kTierCertDD) tor_cert_rho_dd(sigma, dmin2, n, rho, lane);
+    else tor_cert_rho(sigma, dmin2, n, rho, lane);
   }
+  S val = ts_make(0.0, S{});
+  double aux = 0.0;
+  bool ok = true;
+  if (proved) {
+    const unsigned long long subs = 1ull << (n - f - d.param);
+    for (unsigned long long p = 0; p < w.count * subs; ++p) {
+      // pattern over the first n - f modes: the item's own bits lowest
+      const uint32_t pat = (uint32_t)((w.lo + p / subs) | ((p % subs) << d.param));
+      S t = ts_make(0.0, S{});
+      double a = 0.0;
+      ok = tor_rec_item<S, AUX>(Oc, n, n - f, pat, ws, R, rho, lane, t, a) && ok;
+      if (p == 0) {
+        val = t;
+        aux = a;
+      } else {
+        val = ts_add(val, t);
+        if (AUX == 2) aux = ru_add(ru_add(aux, a), ts_sum_err(val));
+        else aux += a;
+      }
+    }
+  }
+  if constexpr (TIER == kTierDD || TIER == kTierCertDD) r.val = ddc{val, dd_make(0.0)};
+  else r.val = ddc{dd_make(val), dd_make(0.0)};
+  r.aux = aux;
+  if (!proved || !ok) r.st = CERT ? kStUncertified : kStOffDomain;
+  __syncwarp();
+  return r;
 }
 
 // ------------------------------------------------------------------ the item kernel

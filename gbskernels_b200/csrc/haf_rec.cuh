@@ -30,12 +30,12 @@
 //     2 (T + 2) accumulators are independent chains, so one or two warps per scheduler
 //     suffice.  T is a template parameter: a rolled loop (Horner's rule, P <- z P + a v)
 //     spent as many register moves as FMAs on the shift
+//     (measured, complex 28 x 28, 256 instances: 19 us each, 33 us rolled, 47 us with a
+//     branch instead of an address select around every load; 250 us by power traces);
 //   * coefficient-major planes [c][pair] with pair index j(j-1)/2 + k, the pair taken
 //     next being the two highest vertices: leaving a pair out is a view (shorter
 //     planes), the operands of a lane are rows of the two taken vertices (contiguous
 //     in k, broadcast in j);
-//     (measured, complex 28 x 28, 256 instances: 19 us each, 33 us rolled, 47 us with a
-//     branch instead of an address select around every load; 250 us by power traces);
 //   * the highest n - m0 pairs are a fixed pattern per block (one state, taken in
 //     place of the former), the next m0 - 5 a depth-first walk, and the last 5 pairs
 //     are walked breadth-first, so that the small states of up to 16 siblings fill the

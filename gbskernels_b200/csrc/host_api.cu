@@ -31,8 +31,7 @@
 #include "haf_pt.cuh"
 #include "haf_rec.cuh"
 #include "tor_lu.cuh"
-#include "tor_warp.cuh"
-#include "tor_warp_dd.cuh"
+#include "tor_rec.cuh"
 
 namespace gbsb {
 
@@ -182,7 +181,7 @@ static double item_cost(int fn, int dim, unsigned long long count, int tier, int
         c = (double)count * dim * dim * dim;
         break;
       }
-      const int qd = n - std::min(n, kTorTailDD);
+      const int qd = n - std::min(n, 4);
       c = (tier == kTierDD || tier == kTierCertDD) ? 20.0 * (double)count * std::ldexp(1.0, qd - param) * 16.0 * (36.0 * qd + 900.0)
                           : (double)count * std::ldexp(1.0, q - param) * 32.0 * (36.0 * q + 1400.0);
       break;
@@ -240,7 +239,7 @@ static int plan_instance(Plan& P, int fn, int tier, int dim_eval, bool real_in, 
     d.param = -1;
   } else if (tier == kTierDD || tier == kTierCertDD) {  // tor, double-double: the warp walk, 16-subset tail
     const int n = dim_eval / 2;
-    const int q = n - std::min(n, kTorTailDD);
+    const int q = n - std::min(n, 4);
     int g = std::max(0, q - 6);  // 2^6 prefix leaves per item
     const int tl = tuned_split(fn, tier, dim_eval);
     if (tl >= 0) g = std::max(0, q - tl);
@@ -285,8 +284,8 @@ static int ws_for_plan(const Plan& P) {
     int w = 0;
     if (fn == kFnPerm) w = 2 * d.dim * d.dim;
     else if (fn == kFnTor && !d.real_in) w = tor_lu_ws_doubles(tier == kTierCert);
-    else if (fn == kFnTor && (tier == kTierDD || tier == kTierCertDD)) w = tor_d_layout(d.dim / 2, tier == kTierCertDD).total;
-    else if (fn == kFnTor) w = tor_w_layout(d.dim / 2, tier == kTierCert).total;
+    else if (fn == kFnTor)
+      w = tor_rec_ws(d.dim / 2, d.param, tier == kTierDD || tier == kTierCertDD, tier_certified(tier));
     else if (tier == kTierDD || tier == kTierCertDD) w = haf_dd_layout(P.haf_smax, tier == kTierCertDD).total;
     else {
       w = rec_ws(d.dim / 2, fn == kFnLhaf, d.real_in);
