@@ -46,6 +46,7 @@ _GPU_MAX_DIM = {
     "lhaf": 32, "lhaf_dd": 32,
     "tor": 48, "tor_dd": 48,
 }
+_C128 = np.dtype(np.complex128)
 _TOR_COMPLEX_MAX_DIM = 24  # complex O (subset LU path), the reference's GPU cap
 
 
@@ -61,7 +62,12 @@ def _check_backend(backend: str) -> None:
 
 
 def _as_stack(matrices: Iterable[Any]) -> np.ndarray:
-    stack = np.ascontiguousarray(np.asarray(matrices, dtype=np.complex128))
+    """The batch as a C-contiguous (B, d, d) array: float64 for real input (the library
+    takes it as it is), complex128 otherwise."""
+    arr = np.asarray(matrices)
+    real = arr.dtype.kind in "fiub" and arr.dtype.itemsize <= 8
+    stack = np.ascontiguousarray(arr if real else np.asarray(matrices, dtype=np.complex128),
+                                 dtype=np.float64 if real else np.complex128)
     if stack.ndim != 3 or stack.shape[1] != stack.shape[2]:
         raise ValueError(
             "GPU backend needs a uniform (B, d, d) stack of square matrices; "
@@ -85,7 +91,7 @@ def _prepare(func: str, matrices: Iterable[Any], precision: str) -> np.ndarray:
     if deff > _GPU_MAX_DIM[name]:
         raise ValueError(f"GPU {name}: matrix dimension {d} exceeds the kernel's limit "
                          f"{_GPU_MAX_DIM[name]}")
-    if func == "tor" and stack.size and float(np.max(np.abs(stack.imag))) > 0.0:
+    if _is_complex_tor(func, stack):
         if precision == "dd":
             raise ValueError("GPU torontonian (precision='dd') is real-domain only; the input "
                              "has non-zero imaginary parts.")
@@ -96,7 +102,7 @@ def _prepare(func: str, matrices: Iterable[Any], precision: str) -> np.ndarray:
 
 
 def _is_complex_tor(func: str, stack: np.ndarray) -> bool:
-    return func == "tor" and stack.size > 0 and float(np.max(np.abs(stack.imag))) > 0.0
+    return func == "tor" and stack.dtype == _C128 and stack.size > 0 and float(np.max(np.abs(stack.imag))) > 0.0
 
 
 def _kernel_dim(func: str, d: int) -> int:
@@ -108,6 +114,11 @@ def _call_uniform(func: str, stack: np.ndarray, precision: str) -> np.ndarray:
     B, d = stack.shape[0], stack.shape[1]
     out = np.empty(B, dtype=np.complex128)
     if B == 0:
+        return out
+    if stack.dtype != _C128:
+        name = "gbs_uniform_real_host"
+        _lib.check(lib.gbs_uniform_real_host(_FN[func], _TIER[precision], _lib.dptr(stack), d, B,
+                                             _lib.dptr(out.view(np.float64))), name)
         return out
     name = f"gbs_{func}_host" if precision == "fp64" else f"gbs_{func}_dd_host"
     fn = getattr(lib, name)
@@ -143,13 +154,15 @@ def _auto_batched(func: str, matrices, return_diagnostics: bool):
     kappa = np.empty(B, dtype=np.float64)
     tier = np.zeros(B, dtype=np.int32)
     if B:
-        rc = _lib.load().gbs_auto_host(_FN[func], _lib.dptr(stack.view(np.float64)), d, B, _AUTO_KAPPA_MAX,
-                                       _lib.dptr(out.view(np.float64)), _lib.dptr(kappa), _lib.iptr(tier))
+        lib = _lib.load()
+        fn = lib.gbs_auto_host if stack.dtype == _C128 else lib.gbs_auto_real_host
+        rc = fn(_FN[func], _lib.dptr(stack.view(np.float64)), d, B, _AUTO_KAPPA_MAX,
+                _lib.dptr(out.view(np.float64)), _lib.dptr(kappa), _lib.iptr(tier))
         # a complex torontonian whose indicator asks for the (real-domain) dd rerun
         _raise_for(rc, f"precision='auto' {func}")
     if not return_diagnostics:
         return out
-    return out, [{"tier": ("fp64", "dd")[t], "cancellation": float(k)} for t, k in zip(tier, kappa)]
+    return out, [{"tier": ("fp64", "dd")[t], "cancellation": k} for t, k in zip(tier.tolist(), kappa.tolist())]
 
 
 def _certified_batched(func: str, matrices, rtol: float | None):
@@ -163,10 +176,10 @@ def _certified_batched(func: str, matrices, rtol: float | None):
     bound = np.empty(B, dtype=np.float64)
     tier = np.zeros(B, dtype=np.int32)
     if B:
-        rc = _lib.load().gbs_certified_ladder_host(_FN[func], _lib.dptr(stack.view(np.float64)), d, B,
-                                                   -1.0 if rtol is None else float(rtol),
-                                                   _lib.dptr(out.view(np.float64)), _lib.dptr(bound),
-                                                   _lib.iptr(tier))
+        lib = _lib.load()
+        fn = lib.gbs_certified_ladder_host if stack.dtype == _C128 else lib.gbs_certified_ladder_real_host
+        rc = fn(_FN[func], _lib.dptr(stack.view(np.float64)), d, B, -1.0 if rtol is None else float(rtol),
+                _lib.dptr(out.view(np.float64)), _lib.dptr(bound), _lib.iptr(tier))
         _raise_for(rc, f"certified {func}", unsupported=NotImplementedError)
     bad = np.flatnonzero(tier < 0)
     if bad.size:
@@ -178,13 +191,12 @@ def _certified_batched(func: str, matrices, rtol: float | None):
     mag = np.abs(out)
     with np.errstate(divide="ignore", invalid="ignore"):
         rel = np.where(mag > 0, bound / np.where(mag > 0, mag, 1.0), np.where(bound == 0, 0.0, np.inf))
-    diags = []
-    for t, e, r in zip(tier, bound, rel):
-        dg = {"tier": "certified-dd" if t == _TIER["certified-dd"] else "certified-fp64",
-              "abs_error_bound": float(e), "rel_error_bound": float(r)}
-        if rtol is not None:
-            dg["escalated"] = bool(t == _TIER["certified-dd"])
-        diags.append(dg)
+    dd = _TIER["certified-dd"]
+    diags = [{"tier": "certified-dd" if t == dd else "certified-fp64", "abs_error_bound": e, "rel_error_bound": r}
+             for t, e, r in zip(tier.tolist(), bound.tolist(), rel.tolist())]
+    if rtol is not None:
+        for dg, t in zip(diags, tier.tolist()):
+            dg["escalated"] = t == dd
     return out, diags
 
 
@@ -541,7 +553,6 @@ def _pack(mats: list[np.ndarray]) -> tuple[np.ndarray, np.ndarray, np.ndarray]:
     return buf, dims, offsets
 
 
-_C128 = np.dtype(np.complex128)
 try:  # the batch walk in C (built beside the library); the Python loop below otherwise
     from . import _hostptr
 except ImportError:
@@ -665,13 +676,13 @@ class Workspace:
             del keep
             _raise_for(rc, f"Workspace.{func}_batched")
             return out
-        mats = _as_square_list(mats)
-        buf, dims, offs = _pack(mats)
+        ptr, dims, keep = _pointers(mats)
         kappa = np.empty(B)
         tier = np.zeros(B, dtype=np.int32)
-        rc = lib.gbs_queue_evaluate_auto(self._session, B, _lib.iptr(fns), _lib.iptr(dims), _lib.llptr(offs),
-                                         _lib.dptr(buf.view(np.float64)), _AUTO_KAPPA_MAX,
-                                         _lib.dptr(out.view(np.float64)), _lib.dptr(kappa), _lib.iptr(tier), None)
+        rc = lib.gbs_queue_evaluate_auto_ptrs(self._session, B, _lib.iptr(fns), _lib.iptr(dims),
+                                              ctypes.c_void_p(ptr.ctypes.data), _AUTO_KAPPA_MAX,
+                                              _lib.dptr(out.view(np.float64)), _lib.dptr(kappa), _lib.iptr(tier), None)
+        del keep
         _raise_for(rc, f"Workspace.{func}_batched")
         return out
 
@@ -689,8 +700,8 @@ class Workspace:
 
     def _call_ptrs(self, funcs, mats, precisions, out, aux, st) -> None:
         ptr, dims, keep = _pointers(mats)
-        fns = np.array([_FN[f] for f in funcs], dtype=np.int32)
-        tiers = np.array([_TIER[p] for p in precisions], dtype=np.int32)
+        fns = np.fromiter(map(_FN.__getitem__, funcs), dtype=np.int32, count=len(funcs))
+        tiers = np.fromiter(map(_TIER.__getitem__, precisions), dtype=np.int32, count=len(precisions))
         rc = _lib.load().gbs_queue_evaluate_ptrs(
             self._session, len(mats), _lib.iptr(fns), _lib.iptr(tiers), _lib.iptr(dims),
             ctypes.c_void_p(ptr.ctypes.data), 0 if self._persistent else 1,
@@ -740,7 +751,7 @@ class Workspace:
             uniform = False
         if not uniform:
             raise ValueError("device-resident output of a ragged batch: use Workspace.evaluate_resident")
-        stack = _prepare(func, stack, "dd" if precision == "dd" else "fp64")
+        _prepare(func, stack, "dd" if precision == "dd" else "fp64")
         if precision == "auto" and _is_complex_tor(func, stack):
             raise NotImplementedError("auto torontonian of a complex O: the double-double rerun is "
                                       "real-domain only; use precision='fp64'")

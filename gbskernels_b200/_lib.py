@@ -34,6 +34,13 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     # value + certified double-double bound
     **{f"gbs_{f}_dd_certified_host": ([_dp, ctypes.c_int, ctypes.c_int, _dp, _dp], ctypes.c_int)
        for f in ("perm", "haf", "lhaf", "tor")},
+    "gbs_uniform_real_host": ([ctypes.c_int, ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, _dp], ctypes.c_int),
+    "gbs_auto_real_host": ([ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, ctypes.c_double, _dp, _dp, _ip],
+                           ctypes.c_int),
+    "gbs_certified_ladder_real_host": ([ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, ctypes.c_double, _dp, _dp,
+                                        _ip], ctypes.c_int),
+    "gbs_queue_evaluate_auto_ptrs": ([_vp, ctypes.c_int, _ip, _ip, _vp, ctypes.c_double, _dp, _dp, _ip, _ip],
+                                     ctypes.c_int),
     "gbs_auto_host": ([ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, ctypes.c_double, _dp, _dp, _ip],
                       ctypes.c_int),
     "gbs_certified_ladder_host": ([ctypes.c_int, _dp, ctypes.c_int, ctypes.c_int, ctypes.c_double, _dp, _dp, _ip],

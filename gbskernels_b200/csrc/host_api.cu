@@ -109,6 +109,7 @@ struct Req {
   // least 2^split work items (the reference's `groups`)
   int single = 0;
   int split = -1;
+  int real_src = 0;  // mat holds dim x dim real numbers (no imaginary parts to look at)
 };
 
 // Device gather of resident-state submatrices (k_gather.cu).
@@ -136,11 +137,11 @@ struct ScatterArgs {
   int write_aux;
 };
 cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st);
+cudaError_t launch_expand_real(const double* in, double* out, long long n, cudaStream_t st);
 
 struct Plan {
   std::vector<InstDesc> insts;
   std::vector<WorkItem> items;
-  std::vector<int> order;
   std::vector<int> trivial;      // instances answered on the host (size-0 / odd haf)
   std::vector<cplx> trivial_val;
   unsigned need = 0;
@@ -168,27 +169,71 @@ static int tuned_warps(int fn, int tier, int dim) {
   return g_tune_warps[fn][(tier == kTierDD || tier == kTierCertDD) ? 1 : 0][dim].load();
 }
 
-// Cost model (relative units) used only to order the queue heaviest-first.
-static double item_cost(int fn, int dim, unsigned long long count, int tier, int param) {
+// How an instance is cut: `nitems` items of `count` subsets / Gray indices / patterns each
+// (the last one may be cut short by `total`), and the InstDesc parameter.
+struct Split {
+  unsigned long long count = 1, total = 1;
+  int param = 0;
+};
+static Split split_of(int fn, int tier, int dim_eval, bool real_in, int split) {
+  Split S;
+  const bool is_dd = tier == kTierDD || tier == kTierCertDD;
+  const int tl = tuned_split(fn, tier, dim_eval);
+  if (fn == kFnPerm) {
+    const int n = dim_eval;
+    S.total = 1ull << (n - 1);
+    if (S.total <= 32) {
+      S.count = S.total;
+    } else {
+      const int rcap = is_dd ? 6 : 10;  // the dd tiers share one split
+      int rlog = std::min(n - 1 - 5, rcap);
+      if (tl >= 0) rlog = std::min(n - 1 - 5, tl);
+      S.count = 32ull << rlog;
+      S.param = rlog;
+    }
+  } else if (fn == kFnHaf || fn == kFnLhaf) {
+    const int n = dim_eval / 2;
+    S.total = 1ull << n;
+    // masks per item: 2^kHafItemLog2 (binary64 tiers) / 2^6 (double-double); smaller instances are one item
+    int per = is_dd ? std::min(n, 6) : std::min(n, kHafItemLog2);  // dd tiers: one split
+    if (tl >= 0) per = std::min(n, tl);
+    S.count = 1ull << per;
+  } else if (!real_in) {  // tor, complex O: ranges of subset masks, one LU per subset
+    const int n = dim_eval / 2;
+    S.total = 1ull << n;
+    S.count = 1ull << std::min(n, 6);
+    S.param = -1;
+  } else {  // tor: one warp per pattern over the first g modes (tor_rec.cuh)
+    const int n = dim_eval / 2;
+    // double-double 2^10 subsets per item; binary64 2^14, the same split for every
+    // binary64 tier so that the certified and indicator values are the fp64 value bit for
+    // bit; a tuned split counts from the last 4 (5) modes
+    const int q = n - std::min(n, is_dd ? 4 : 5);
+    int g = std::max(0, q - (is_dd ? 6 : 9));
+    if (tl >= 0) g = std::max(0, q - tl);
+    if (split >= 0 && !is_dd) g = std::min(q, std::max(g, split));
+    S.total = 1ull << g;
+    S.count = 1;
+    S.param = g;
+  }
+  return S;
+}
+
+// Cost model (instructions of a lane) used only to order the queue heaviest-first.
+static double item_cost(int fn, int dim, int tier, const Split& S) {
+  const double count = (double)S.count, n = dim / 2.0;
+  const bool is_dd = tier == kTierDD || tier == kTierCertDD;
   double c;
   switch (fn) {
-    case kFnPerm: c = (double)count * dim; break;
-    case kFnTor: {
-      // binary64 tiers: count prefix patterns, 2^(q - g) leaves of 32 subsets each
-      // (g = param); double-double: count lanes of 2^(n - g) subsets each
-      const int n = dim / 2, q = n - std::min(n, 5);
-      if (param < 0) {  // complex O: count subset LU factorisations
-        c = (double)count * dim * dim * dim;
-        break;
-      }
-      const int qd = n - std::min(n, 4);
-      c = (tier == kTierDD || tier == kTierCertDD) ? 20.0 * (double)count * std::ldexp(1.0, qd - param) * 16.0 * (36.0 * qd + 900.0)
-                          : (double)count * std::ldexp(1.0, q - param) * 32.0 * (36.0 * q + 1400.0);
+    case kFnPerm: c = count * dim * 6.0; break;
+    case kFnTor:
+      c = S.param < 0 ? count * dim * dim * dim : count * std::ldexp(120.0, dim / 2 - S.param);
       break;
-    }
-    default: { double n = dim / 2.0; c = (double)count * (n + 1) * n * n * n; break; }
+    default:  // recursion over pairs; the indicator and the double-double tiers run power traces
+      c = count * 12.0 * n * n * (fn == kFnLhaf ? 1.9 : 1.0);
+      if (tier == kTierKappa || is_dd) c += count * (n + 1) * n * n * n;
   }
-  return (tier == kTierDD || tier == kTierCertDD) ? 20.0 * c : c;
+  return is_dd ? 20.0 * c : c;
 }
 
 // Append one instance (already validated) to the plan.  Returns the instance index.
@@ -201,62 +246,16 @@ static int plan_instance(Plan& P, int fn, int tier, int dim_eval, bool real_in, 
   d.param = 0;
   d.real_in = real_in ? 1 : 0;
   const int idx = (int)P.insts.size();
-  auto add = [&](unsigned long long lo, unsigned long long count) {
+  const Split S = split_of(fn, tier, dim_eval, real_in, split);
+  d.param = S.param;
+  for (unsigned long long lo = 0; lo < S.total; lo += S.count) {
     WorkItem w{};
     w.inst = idx;
     w.lo = lo;
-    w.count = count;
+    w.count = std::min(S.count, S.total - lo);
     P.items.push_back(w);
-  };
-  if (fn == kFnPerm) {
-    const int n = dim_eval;
-    const unsigned long long terms = 1ull << (n - 1);
-    if (terms <= 32) {
-      add(0, terms);
-    } else {
-      const int rcap = (tier == kTierDD || tier == kTierCertDD) ? 6 : 10;  // the dd tiers share one split
-      int rlog = std::min(n - 1 - 5, rcap);
-      const int tl = tuned_split(fn, tier, dim_eval);
-      if (tl >= 0) rlog = std::min(n - 1 - 5, tl);
-      const unsigned long long cnt = 32ull << rlog;
-      for (unsigned long long lo = 0; lo < terms; lo += cnt) add(lo, cnt);
-      d.param = rlog;
-    }
-  } else if (fn == kFnHaf || fn == kFnLhaf) {
-    const int n = dim_eval / 2;
-    const unsigned long long masks = 1ull << n;
-    // masks per item: 2^kHafItemLog2 (binary64 tiers) / 2^6 (double-double); smaller instances are one item
-    int per = (tier == kTierDD || tier == kTierCertDD) ? std::min(n, 6) : std::min(n, kHafItemLog2);  // dd tiers: one split
-    const int tl = tuned_split(fn, tier, dim_eval);
-    if (tl >= 0) per = std::min(n, tl);
-    const unsigned long long cnt = 1ull << per;
-    for (unsigned long long lo = 0; lo < masks; lo += cnt) add(lo, std::min(cnt, masks - lo));
-    P.haf_smax = std::max(P.haf_smax, dim_eval);
-  } else if (!real_in) {  // tor, complex O: ranges of subset masks, one LU per subset
-    const int n = dim_eval / 2;
-    const int per = std::min(n, 6);
-    for (unsigned long long lo = 0; lo < (1ull << n); lo += (1ull << per)) add(lo, 1ull << per);
-    d.param = -1;
-  } else if (tier == kTierDD || tier == kTierCertDD) {  // tor, double-double: the warp walk, 16-subset tail
-    const int n = dim_eval / 2;
-    const int q = n - std::min(n, 4);
-    int g = std::max(0, q - 6);  // 2^6 prefix leaves per item
-    const int tl = tuned_split(fn, tier, dim_eval);
-    if (tl >= 0) g = std::max(0, q - tl);
-    for (unsigned long long p = 0; p < (1ull << g); ++p) add(p, 1);
-    d.param = g;
-  } else {  // tor, binary64 tiers: one warp per prefix pattern over the first g prefix modes
-    const int n = dim_eval / 2;
-    const int q = n - std::min(n, 5);
-    // 2^9 leaves (x 32 tail subsets) per item, the same split for every binary64
-    // tier so that the certified and indicator values are the fp64 value bit for bit
-    int g = std::max(0, q - 9);
-    const int tl = tuned_split(fn, tier, dim_eval);  // log2 prefix leaves per item
-    if (tl >= 0) g = std::max(0, q - tl);
-    if (split >= 0) g = std::min(q, std::max(g, split));
-    for (unsigned long long p = 0; p < (1ull << g); ++p) add(p, 1);
-    d.param = g;
   }
+  if (fn == kFnHaf || fn == kFnLhaf) P.haf_smax = std::max(P.haf_smax, dim_eval);
   d.nitems = (int)P.items.size() - d.item0;
   P.insts.push_back(d);
   P.need |= 1u << d.ft;
@@ -306,6 +305,8 @@ struct PinBuf {
   void* p = nullptr;
   size_t cap = 0;
 };
+// results of a plan, per instance: complex value, aux, status (each array contiguous)
+constexpr size_t kResultBytes = 3 * sizeof(double) + sizeof(int);
 
 }  // namespace gbsb
 
@@ -313,8 +314,9 @@ struct gbs_session {
   cudaStream_t stream = nullptr;
   int device = 0;
   int sms = 148;
-  gbsb::DevBuf mats, meta, part, paux, pst, done, head, out, aux, st;
-  gbsb::PinBuf pin_in, pin_meta, pin_out;
+  gbsb::DevBuf mats, part, paux, pst, head, out;
+  gbsb::DevBuf real;       // a real batch as uploaded, before it is widened to complex
+  gbsb::PinBuf pin_in, pin_out;
   gbsb::DevBuf gather;
   gbsb::PinBuf pin_gather;
   gbsb::DevBuf rmap;       // instance -> request map and trivial values of a resident read
@@ -391,6 +393,7 @@ static cudaError_t grow_pin(PinBuf& b, size_t bytes) {
 static bool haf_real_path(const Req& r) {
   if (r.state || !r.mat) return false;
   if (r.tier != kTierFp64 && r.tier != kTierKappa && r.tier != kTierCert) return false;
+  if (r.real_src) return true;
   const size_t nn = (size_t)r.dim * r.dim;
   for (size_t i = 0; i < nn; ++i)
     if (r.mat[2 * i + 1] != 0.0) return false;
@@ -437,7 +440,7 @@ static int check_req(const Req& r, int* dim_eval, bool* real_in, bool* trivial, 
       bool re = true;
       if (r.state) {
         re = r.state_real != 0;
-      } else {
+      } else if (!r.real_src) {
         const size_t nn = (size_t)r.dim * r.dim;
         for (size_t i = 0; i < nn; ++i)
           if (r.mat[2 * i + 1] != 0.0) { re = false; break; }
@@ -543,46 +546,59 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
   size_t meta_bytes = 0, tot_items = 0, tot_inst = 0;
   for (size_t g = 0; g < plans.size(); ++g) {
     Plan& P = plans[g];
+    // heaviest instances first: the queue is pulled in item order
+    if (opt.sort_heavy && !opt.per_size) {
+      std::vector<std::pair<double, int>> c;
+      c.reserve(greq[g].size());
+      size_t nit = 0;
+      for (int i : greq[g]) {
+        const Split S = split_of(reqs[i].fn, reqs[i].tier, dim_eval[i], real_in[i], reqs[i].split);
+        nit += (size_t)((S.total + S.count - 1) / S.count);
+        c.emplace_back(-item_cost(reqs[i].fn, dim_eval[i], reqs[i].tier, S), i);
+      }
+      std::stable_sort(c.begin(), c.end(), [](auto& a, auto& b) { return a.first < b.first; });
+      for (size_t k = 0; k < c.size(); ++k) greq[g][k] = c[k].second;
+      P.items.reserve(nit);
+      P.insts.reserve(c.size());
+    }
     for (int i : greq[g]) plan_instance(P, reqs[i].fn, reqs[i].tier, dim_eval[i], real_in[i], off[i], reqs[i].split);
     P.ws_doubles = ws_for_plan(P);
     const int ni = (int)P.insts.size(), nit = (int)P.items.size();
-    std::vector<int> inst_order(ni);
-    for (int k = 0; k < ni; ++k) inst_order[k] = k;
-    if (opt.sort_heavy && !opt.per_size) {
-      std::vector<double> c(ni);
-      for (int k = 0; k < ni; ++k) {
-        const InstDesc& d = P.insts[k];
-        c[k] = item_cost(ft_fn(d.ft), d.dim, P.items[d.item0].count, ft_tier(d.ft), d.param);
-      }
-      std::stable_sort(inst_order.begin(), inst_order.end(), [&](int a, int b) { return c[a] > c[b]; });
-    }
-    P.order.reserve(nit);
-    for (int k : inst_order)
-      for (int j = 0; j < P.insts[k].nitems; ++j) P.order.push_back(P.insts[k].item0 + j);
     if (cover(P.need) == 0) return fail(cudaErrorNotSupported, "no compiled kernel covers this mix");
-    meta_bytes += ((ni * sizeof(InstDesc) + nit * sizeof(WorkItem) + nit * sizeof(int)) + 255) & ~(size_t)255;
+    meta_bytes += ((ni * sizeof(InstDesc) + nit * sizeof(WorkItem)) + 255) & ~(size_t)255;
     tot_items += nit;
     tot_inst += ni;
   }
   // ---- buffers (monotone growth)
-  cudaError_t e = grow_pin(s->pin_in, std::max<long long>(mat_doubles, 2) * sizeof(double));
-  if (e == cudaSuccess) e = grow_dev(s->mats, std::max<long long>(mat_doubles, 2) * sizeof(double), &s->reallocs);
-  if (e == cudaSuccess) e = grow_pin(s->pin_meta, std::max<size_t>(meta_bytes, 256));
-  if (e == cudaSuccess) e = grow_dev(s->meta, std::max<size_t>(meta_bytes, 256), &s->reallocs);
+  // (matrices and queues share a buffer on each side, so that a small batch is one
+  // upload; so do the queue heads and counters, and the results: one reset, one read-back)
+  const size_t mat_bytes = ((size_t)std::max<long long>(mat_doubles, 2) * sizeof(double) + 255) & ~(size_t)255;
+  const size_t heads = 64 * std::max<size_t>(plans.size(), 1), insts1 = std::max<size_t>(tot_inst, 1);
+  cudaError_t e = grow_pin(s->pin_in, mat_bytes + meta_bytes);
+  if (e == cudaSuccess) e = grow_dev(s->mats, mat_bytes + meta_bytes, &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->part, std::max<size_t>(tot_items, 1) * 4 * sizeof(double), &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->paux, std::max<size_t>(tot_items, 1) * sizeof(double), &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->pst, std::max<size_t>(tot_items, 1) * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->done, std::max<size_t>(tot_inst, 1) * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->head, 64 * std::max<size_t>(plans.size(), 1), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->out, std::max<size_t>(tot_inst, 1) * 2 * sizeof(double), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->aux, std::max<size_t>(tot_inst, 1) * sizeof(double), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->st, std::max<size_t>(tot_inst, 1) * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_pin(s->pin_out, std::max<size_t>(tot_inst, 1) * (3 * sizeof(double) + sizeof(int)));
+  if (e == cudaSuccess) e = grow_dev(s->head, heads + insts1 * sizeof(int), &s->reallocs);
+  if (e == cudaSuccess) e = grow_dev(s->out, insts1 * kResultBytes, &s->reallocs);
+  if (e == cudaSuccess) e = grow_pin(s->pin_out, insts1 * kResultBytes);
   if (e != cudaSuccess) return fail(e, "allocating session buffers");
   // staging buffers may still be read by copies of a previous call
   e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) return fail(e, "synchronising the session stream");
-  // ---- pack matrices (odd loop hafnians augmented by A (+) [1]) and upload once
+  // ---- pack matrices (odd loop hafnians augmented by A (+) [1]) and upload once: with the
+  // queues when that is small and nothing on the device has to read it before, else while
+  // the queues are still being written
+  bool one_upload = mat_bytes + meta_bytes <= (256u << 10);
+  for (int i = 0; i < B && one_upload; ++i) one_upload = !reqs[i].state;
+  // a large batch of real matrices travels as it is and is widened on the device
+  bool real_upload = !one_upload;
+  for (int i = 0; i < B && real_upload; ++i)
+    real_upload = s->plan_trivial[i] || (reqs[i].real_src && dim_eval[i] == reqs[i].dim);
+  if (real_upload && mat_doubles > 0) {
+    e = grow_dev(s->real, (size_t)mat_doubles / 2 * sizeof(double), &s->reallocs);
+    if (e != cudaSuccess) return fail(e, "allocating the real input buffer");
+  }
   {
     double* dst = (double*)s->pin_in.p;
     s->gdesc.clear();
@@ -606,7 +622,19 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
         const int i = host_rows[k];
         const long long o = off[i];
         const int d = reqs[i].dim, de = dim_eval[i];
-        if (de == d) {
+        if (real_upload) {
+          std::memcpy(dst + o / 2, reqs[i].mat, sizeof(double) * (size_t)d * d);
+        } else if (reqs[i].real_src) {
+          const double* src = reqs[i].mat;
+          double* q = dst + o;
+          if (de != d) std::memset(q, 0, sizeof(double) * 2 * (size_t)de * de);
+          for (int r = 0; r < d; ++r)
+            for (int c = 0; c < d; ++c) {
+              q[2 * ((size_t)r * de + c)] = src[(size_t)r * d + c];
+              q[2 * ((size_t)r * de + c) + 1] = 0.0;
+            }
+          if (de != d) q[2ll * ((long long)d * de + d)] = 1.0;
+        } else if (de == d) {
           std::memcpy(dst + o, reqs[i].mat, sizeof(double) * 2 * (size_t)d * d);
         } else {
           std::memset(dst + o, 0, sizeof(double) * 2 * (size_t)de * de);
@@ -619,7 +647,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     // a large batch is packed by several host threads (disjoint ranges of requests,
     // disjoint destination ranges): one thread copies a few GB/s, short of what the
     // upload that follows moves
-    const size_t bytes = (size_t)std::max<long long>(mat_doubles, 0) * sizeof(double);
+    const size_t bytes = (size_t)std::max<long long>(mat_doubles, 0) * sizeof(double) / (real_upload ? 2 : 1);
     const int nth = (int)std::min<size_t>({(size_t)std::max(1u, std::thread::hardware_concurrency()), (size_t)8,
                                             bytes / (8u << 20) + 1, host_rows.size() + 1});
     if (nth <= 1) {
@@ -638,8 +666,14 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
       }
       for (auto& t : th) t.join();
     }
-    if (mat_doubles > 0) {
-      e = cudaMemcpyAsync(s->mats.p, s->pin_in.p, mat_doubles * sizeof(double), cudaMemcpyHostToDevice, s->stream);
+    if (mat_doubles > 0 && !one_upload) {
+      if (real_upload) {
+        e = cudaMemcpyAsync(s->real.p, s->pin_in.p, mat_doubles / 2 * sizeof(double), cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess)
+          e = launch_expand_real((const double*)s->real.p, (double*)s->mats.p, mat_doubles / 2, s->stream);
+      } else {
+        e = cudaMemcpyAsync(s->mats.p, s->pin_in.p, mat_doubles * sizeof(double), cudaMemcpyHostToDevice, s->stream);
+      }
       if (e != cudaSuccess) return fail(e, "uploading matrices");
     }
     if (!s->gdesc.empty()) {
@@ -658,30 +692,28 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
   }
   // ---- queues
   size_t moff = 0, ioff = 0, noff = 0;
-  char* pm = (char*)s->pin_meta.p;
+  char* pm = (char*)s->pin_in.p + mat_bytes;
   for (size_t g = 0; g < plans.size(); ++g) {
     Plan& P = plans[g];
     const int ni = (int)P.insts.size(), nit = (int)P.items.size();
-    // shift item0 of every instance and the order entries to this group's slots
     std::memcpy(pm + moff, P.insts.data(), ni * sizeof(InstDesc));
     std::memcpy(pm + moff + ni * sizeof(InstDesc), P.items.data(), nit * sizeof(WorkItem));
-    std::memcpy(pm + moff + ni * sizeof(InstDesc) + nit * sizeof(WorkItem), P.order.data(), nit * sizeof(int));
     gbs_session::Group G;
     ItemLaunch& L = G.L;
-    char* dm = (char*)s->meta.p + moff;
+    char* dm = (char*)s->mats.p + mat_bytes + moff;
     L.mats = (const double*)s->mats.p;
     L.insts = (const InstDesc*)dm;
     L.items = (const WorkItem*)(dm + ni * sizeof(InstDesc));
-    L.order = (const int*)(dm + ni * sizeof(InstDesc) + nit * sizeof(WorkItem));
+    L.order = nullptr;
     L.n_items = nit;
     L.head = (int*)((char*)s->head.p + 64 * g);
-    L.done = (int*)s->done.p + noff;
+    L.done = (int*)((char*)s->head.p + heads) + noff;
     L.part = (double*)s->part.p + 4 * ioff;
     L.paux = (double*)s->paux.p + ioff;
     L.pst = (int*)s->pst.p + ioff;
     L.out = (double*)s->out.p + 2 * noff;
-    L.aux_out = (double*)s->aux.p + noff;
-    L.st_out = (int*)s->st.p + noff;
+    L.aux_out = (double*)s->out.p + 2 * tot_inst + noff;
+    L.st_out = (int*)((double*)s->out.p + 3 * tot_inst) + noff;
     L.ws_doubles = P.ws_doubles;
     L.haf_smax = P.haf_smax;
     G.br = cover(P.need);
@@ -714,12 +746,14 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     G.out_off = noff;
     G.req = greq[g];
     s->groups.push_back(std::move(G));
-    moff += ((ni * sizeof(InstDesc) + nit * sizeof(WorkItem) + nit * sizeof(int)) + 255) & ~(size_t)255;
+    moff += ((ni * sizeof(InstDesc) + nit * sizeof(WorkItem)) + 255) & ~(size_t)255;
     ioff += nit;
     noff += ni;
   }
   if (moff > 0) {
-    e = cudaMemcpyAsync(s->meta.p, pm, moff, cudaMemcpyHostToDevice, s->stream);
+    const size_t skip = one_upload ? 0 : mat_bytes;
+    e = cudaMemcpyAsync((char*)s->mats.p + skip, (char*)s->pin_in.p + skip, mat_bytes - skip + moff,
+                        cudaMemcpyHostToDevice, s->stream);
     if (e != cudaSuccess) return fail(e, "uploading the work queues");
   }
   s->plan_ninst = noff;
@@ -733,8 +767,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
 static cudaError_t plan_enqueue(gbs_session* s, cudaStream_t stream) {
   cudaError_t e = cudaSuccess;
   if (!s->groups.empty()) {
-    e = cudaMemsetAsync(s->head.p, 0, 64 * s->groups.size(), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->done.p, 0, s->plan_ninst * sizeof(int), stream);
+    e = cudaMemsetAsync(s->head.p, 0, 64 * s->groups.size() + s->plan_ninst * sizeof(int), stream);
   }
   for (auto& G : s->groups) {
     if (e != cudaSuccess) break;
@@ -790,13 +823,9 @@ static int plan_read_enqueue(gbs_session* s, cudaStream_t stream) {
   if (!stream) stream = s->stream;
   const size_t ni = s->plan_ninst;
   double* po = (double*)s->pin_out.p;
-  double* pa = po + 2 * ni;
-  int* ps = (int*)(pa + ni);
   cudaError_t e = cudaSuccess;
   if (ni > 0) {
-    e = cudaMemcpyAsync(po, s->out.p, ni * 2 * sizeof(double), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(pa, s->aux.p, ni * sizeof(double), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ps, s->st.p, ni * sizeof(int), cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(po, s->out.p, ni * kResultBytes, cudaMemcpyDeviceToHost, stream);
   }
   return e == cudaSuccess ? 0 : fail(e, "reading results back");
 }
@@ -865,8 +894,8 @@ static int plan_scatter(gbs_session* s, cudaStream_t stream, double* block, int 
   if (e != cudaSuccess) return fail(e, "uploading the resident result map");
   ScatterArgs a{};
   a.out = (const double*)s->out.p;
-  a.aux = (const double*)s->aux.p;
-  a.st = (const int*)s->st.p;
+  a.aux = (const double*)s->out.p + 2 * (size_t)ni;
+  a.st = (const int*)((const double*)s->out.p + 3 * (size_t)ni);
   a.map = (const int*)s->rmap.p;
   a.ni = ni;
   a.tidx = (const int*)s->rmap.p + ni;
@@ -930,10 +959,9 @@ static void session_free(gbs_session* s) {
   if (!s) return;
   if (s->stream) cudaStreamSynchronize(s->stream);
   drop_graph(s);
-  for (DevBuf* b : {&s->mats, &s->meta, &s->part, &s->paux, &s->pst, &s->done, &s->head, &s->out, &s->aux, &s->st,
-                    &s->gather})
+  for (DevBuf* b : {&s->mats, &s->part, &s->paux, &s->pst, &s->head, &s->out, &s->real, &s->gather, &s->rmap})
     if (b->p) cudaFree(b->p);
-  for (PinBuf* b : {&s->pin_in, &s->pin_meta, &s->pin_out, &s->pin_gather})
+  for (PinBuf* b : {&s->pin_in, &s->pin_out, &s->pin_gather, &s->pin_rmap})
     if (b->p) cudaFreeHost(b->p);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
@@ -951,14 +979,39 @@ static int with_default(gbs_session** s) {
   return 0;
 }
 
+// Requests of a uniform (B, d, d) batch of complex (or, real_src, real) matrices.
+static std::vector<Req> uniform_reqs(int fn, int tier, const double* m, int dim, int b, bool real_src) {
+  std::vector<Req> reqs(b);
+  const size_t stride = (real_src ? 1ull : 2ull) * dim * dim;
+  for (int i = 0; i < b; ++i) {
+    reqs[i] = Req{fn, tier, dim, m + i * stride};
+    reqs[i].real_src = real_src ? 1 : 0;
+  }
+  return reqs;
+}
+
+// Whether every number is finite (no early exit inside a block, so that it vectorises).
+static bool all_finite(const double* m, size_t n) {
+  constexpr unsigned long long kExp = 0x7ff0000000000000ull;
+  for (size_t i = 0; i < n; i += 4096) {
+    const size_t e = std::min(n, i + 4096);
+    unsigned long long bad = 0;
+    for (size_t k = i; k < e; ++k) {
+      unsigned long long x;
+      std::memcpy(&x, m + k, 8);
+      bad |= (unsigned long long)((x & kExp) == kExp);
+    }
+    if (bad) return false;
+  }
+  return true;
+}
+
 // Uniform (B, d, d) batch through a session.
 static int uniform(gbs_session* s, int fn, int tier, const double* m, int dim, int b, double* o, double* aux,
-                   int* st) {
+                   int* st, bool real_src = false) {
   if (b <= 0) return 0;
   if (!m || !o) return fail(cudaErrorInvalidValue, "null buffer");
-  std::vector<Req> reqs(b);
-  const size_t stride = 2ull * dim * dim;
-  for (int i = 0; i < b; ++i) reqs[i] = Req{fn, tier, dim, m + i * stride};
+  const std::vector<Req> reqs = uniform_reqs(fn, tier, m, dim, b, real_src);
   std::lock_guard<std::mutex> lk(s->mu);
   RunOpts opt;
   return run_batch(s, reqs, o, aux, st, opt);
@@ -970,12 +1023,13 @@ static void apply_status(int b, double* o, const int* st) {
     if (st[i] != kStOk) { o[2 * i] = NAN; o[2 * i + 1] = NAN; }
 }
 
-static int one_shot(int fn, int tier, const double* m, int dim, int b, double* o, double* aux) {
+static int one_shot(int fn, int tier, const double* m, int dim, int b, double* o, double* aux,
+                    bool real_src = false) {
   gbs_session* s;
   int rc = with_default(&s);
   if (rc) return rc;
   std::vector<int> st(std::max(b, 0));
-  rc = uniform(s, fn, tier, m, dim, b, o, aux, st.data());
+  rc = uniform(s, fn, tier, m, dim, b, o, aux, st.data(), real_src);
   if (rc == 0) apply_status(b, o, st.data());
   return rc;
 }
@@ -1027,20 +1081,15 @@ static int auto_batch(gbs_session* s, const std::vector<Req>& reqs, double kappa
 static int session_reserve(gbs_session* s, size_t mat_bytes, size_t items, size_t insts) {
   items = std::max<size_t>(items, 1);
   insts = std::max<size_t>(insts, 1);
-  const size_t meta = insts * sizeof(InstDesc) + items * (sizeof(WorkItem) + sizeof(int)) + 1024;
-  cudaError_t e = grow_pin(s->pin_in, std::max<size_t>(mat_bytes, 16));
-  if (e == cudaSuccess) e = grow_dev(s->mats, std::max<size_t>(mat_bytes, 16), &s->reallocs);
-  if (e == cudaSuccess) e = grow_pin(s->pin_meta, meta);
-  if (e == cudaSuccess) e = grow_dev(s->meta, meta, &s->reallocs);
+  const size_t in = std::max<size_t>(mat_bytes, 16) + insts * sizeof(InstDesc) + items * sizeof(WorkItem) + 1024;
+  cudaError_t e = grow_pin(s->pin_in, in);
+  if (e == cudaSuccess) e = grow_dev(s->mats, in, &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->part, items * 4 * sizeof(double), &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->paux, items * sizeof(double), &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->pst, items * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->done, insts * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->head, 64 * 8, &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->out, insts * 2 * sizeof(double), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->aux, insts * sizeof(double), &s->reallocs);
-  if (e == cudaSuccess) e = grow_dev(s->st, insts * sizeof(int), &s->reallocs);
-  if (e == cudaSuccess) e = grow_pin(s->pin_out, insts * (3 * sizeof(double) + sizeof(int)));
+  if (e == cudaSuccess) e = grow_dev(s->head, 64 * 8 + insts * sizeof(int), &s->reallocs);
+  if (e == cudaSuccess) e = grow_dev(s->out, insts * kResultBytes, &s->reallocs);
+  if (e == cudaSuccess) e = grow_pin(s->pin_out, insts * kResultBytes);
   return e == cudaSuccess ? 0 : fail(e, "reserving the session buffers");
 }
 
@@ -1149,11 +1198,12 @@ int gbs_lhaf_kappa_host(const double* m, int N, int b, double* o, double* a) { r
 int gbs_tor_kappa_host(const double* m, int n, int b, double* o, double* a) { return one_shot(kFnTor, kTierKappa, m, 2 * n, b, o, a); }
 
 // ---- certified tier: value + rigorous bound (core/host_api.cu:248-262) ---------
-static int one_shot_cert(int fn, const double* m, int dim, int b, double* o, double* bound, int tier = kTierCert) {
+static int one_shot_cert(int fn, const double* m, int dim, int b, double* o, double* bound, int tier = kTierCert,
+                         bool real_src = false) {
   if (b > 0 && !bound) return fail(cudaErrorInvalidValue, "null bound buffer");
-  for (size_t i = 0; i < 2ull * (size_t)dim * dim * (size_t)std::max(b, 0); ++i)
-    if (!std::isfinite(m[i])) return fail(cudaErrorInvalidValue, "certified evaluation requires finite input");
-  int rc = one_shot(fn, tier, m, dim, b, o, bound);
+  if (!all_finite(m, (real_src ? 1ull : 2ull) * (size_t)dim * dim * (size_t)std::max(b, 0)))
+    return fail(cudaErrorInvalidValue, "certified evaluation requires finite input");
+  int rc = one_shot(fn, tier, m, dim, b, o, bound, real_src);
   if (rc == 0)
     for (int i = 0; i < b; ++i)
       if (std::isnan(o[2 * i])) bound[i] = INFINITY;
@@ -1227,21 +1277,35 @@ int gbs_tor_single_ddcertified_host(const double* O, int n, int g, double* out, 
 
 // ---- auto tier on the device (gbskernels/__init__.py:272-297) ----------------
 // func: 0 perm, 1 haf, 2 lhaf, 3 tor; dim = matrix side.  tier_out: 0 fp64, 1 dd.
-int gbs_auto_host(int func, const double* m, int dim, int b, double kappa_max, double* o, double* kappa,
-                  int* tier_out) {
+static int auto_host(int func, const double* m, int dim, int b, double kappa_max, double* o, double* kappa,
+                     int* tier_out, bool real_src) {
   if (b <= 0) return 0;
   if (!m || !o || !tier_out) return fail(cudaErrorInvalidValue, "null buffer");
   gbs_session* s;
   int rc = with_default(&s);
   if (rc) return rc;
-  std::vector<Req> reqs(b);
-  const size_t stride = 2ull * dim * dim;
-  for (int i = 0; i < b; ++i) reqs[i] = Req{func, kTierFp64, dim, m + i * stride};
+  const std::vector<Req> reqs = uniform_reqs(func, kTierFp64, m, dim, b, real_src);
   std::vector<int> st(b);
   std::lock_guard<std::mutex> lk(s->mu);
   rc = auto_batch(s, reqs, kappa_max, o, kappa, tier_out, st.data());
   if (rc == 0) apply_status(b, o, st.data());
   return rc;
+}
+int gbs_auto_host(int func, const double* m, int dim, int b, double kappa_max, double* o, double* kappa,
+                  int* tier_out) {
+  return auto_host(func, m, dim, b, kappa_max, o, kappa, tier_out, false);
+}
+
+// ---- uniform batches of real matrices (B, d, d), dim = matrix side: what the complex entry
+// points give for the same numbers, without the caller widening them and without a look
+// at the imaginary parts.  tier 0 fp64 or 1 double-double.
+int gbs_uniform_real_host(int func, int tier, const double* m, int dim, int b, double* o) {
+  if (tier != kTierFp64 && tier != kTierDD) return fail(cudaErrorInvalidValue, "unsupported precision tier");
+  return one_shot(func, tier, m, dim, b, o, nullptr, true);
+}
+int gbs_auto_real_host(int func, const double* m, int dim, int b, double kappa_max, double* o, double* kappa,
+                       int* tier_out) {
+  return auto_host(func, m, dim, b, kappa_max, o, kappa, tier_out, true);
 }
 
 // ---- certified tier with the proven rtol ladder (gbskernels/__init__.py:374-478) ----
@@ -1259,28 +1323,28 @@ static bool certificate_meets(double re, double im, double e, double rtol) {
   return e / mag <= rtol;
 }
 
-int gbs_certified_ladder_host(int func, const double* m, int dim, int b, double rtol, double* o, double* bound,
-                              int* tier_out) {
+static int certified_ladder(int func, const double* m, int dim, int b, double rtol, double* o, double* bound,
+                            int* tier_out, bool real_src) {
   if (b <= 0) return 0;
   if (!m || !o || !bound || !tier_out) return fail(cudaErrorInvalidValue, "null buffer");
   if (func < kFnPerm || func > kFnTor) return fail(cudaErrorInvalidValue, "unknown function code");
   if (func == kFnTor && (dim & 1)) return fail(cudaErrorInvalidValue, "torontonian: matrix side must be even");
-  int rc = one_shot_cert(func, m, dim, b, o, bound, kTierCert);
+  int rc = one_shot_cert(func, m, dim, b, o, bound, kTierCert, real_src);
   if (rc) return rc;
-  const size_t nn = 2ull * (size_t)dim * dim;
+  const size_t nn = (real_src ? 1ull : 2ull) * (size_t)dim * dim;
   std::vector<int> redo;
   for (int i = 0; i < b; ++i) {
     const bool ok = certificate_meets(o[2 * i], o[2 * i + 1], bound[i], rtol);
     tier_out[i] = ok ? kTierCert : -1;
     bool real = true;  // the double-double torontonian is real-domain only
-    if (func == kFnTor)
+    if (!ok && func == kFnTor && !real_src)
       for (size_t k = 1; k < nn && real; k += 2) real = m[i * nn + k] == 0.0;
     if (!ok && rtol >= 0.0 && real) redo.push_back(i);
   }
   if (redo.empty()) return 0;
   std::vector<double> sub(nn * redo.size()), o2(2 * redo.size()), b2(redo.size());
   for (size_t j = 0; j < redo.size(); ++j) std::memcpy(&sub[j * nn], m + redo[j] * nn, nn * sizeof(double));
-  rc = one_shot_cert(func, sub.data(), dim, (int)redo.size(), o2.data(), b2.data(), kTierCertDD);
+  rc = one_shot_cert(func, sub.data(), dim, (int)redo.size(), o2.data(), b2.data(), kTierCertDD, real_src);
   if (rc) return rc;
   for (size_t j = 0; j < redo.size(); ++j) {
     if (!certificate_meets(o2[2 * j], o2[2 * j + 1], b2[j], rtol)) continue;
@@ -1291,6 +1355,14 @@ int gbs_certified_ladder_host(int func, const double* m, int dim, int b, double 
     tier_out[i] = kTierCertDD;
   }
   return 0;
+}
+int gbs_certified_ladder_host(int func, const double* m, int dim, int b, double rtol, double* o, double* bound,
+                              int* tier_out) {
+  return certified_ladder(func, m, dim, b, rtol, o, bound, tier_out, false);
+}
+int gbs_certified_ladder_real_host(int func, const double* m, int dim, int b, double rtol, double* o, double* bound,
+                                   int* tier_out) {
+  return certified_ladder(func, m, dim, b, rtol, o, bound, tier_out, true);
 }
 
 // ---- sessions (core/host_api.cu:521-658) --------------------------------------
@@ -1440,6 +1512,26 @@ int gbs_queue_evaluate_auto(gbs_session* s, int B, const int* funcs, const int* 
   if (!funcs || !dims || !offsets || !mats || !out || !tier_out) return fail(cudaErrorInvalidValue, "null buffer");
   std::vector<Req> reqs(B);
   for (int i = 0; i < B; ++i) reqs[i] = Req{funcs[i], kTierFp64, dims[i], mats + 2 * offsets[i]};
+  std::vector<int> st(B);
+  std::lock_guard<std::mutex> lk(s->mu);
+  const int rc = auto_batch(s, reqs, kappa_max, out, kappa, tier_out, st.data());
+  if (rc) return rc;
+  if (status) std::memcpy(status, st.data(), sizeof(int) * B);
+  apply_status(B, out, st.data());
+  return 0;
+}
+
+// As gbs_queue_evaluate_auto, with one host pointer per matrix.
+int gbs_queue_evaluate_auto_ptrs(gbs_session* s, int B, const int* funcs, const int* dims, const double* const* mats,
+                                 double kappa_max, double* out, double* kappa, int* tier_out, int* status) {
+  if (!s) return fail(cudaErrorInvalidValue, "null session");
+  if (B <= 0) return 0;
+  if (!funcs || !dims || !mats || !out || !tier_out) return fail(cudaErrorInvalidValue, "null buffer");
+  std::vector<Req> reqs(B);
+  for (int i = 0; i < B; ++i) {
+    if (!mats[i] && dims[i] > 0) return fail(cudaErrorInvalidValue, "null matrix pointer");
+    reqs[i] = Req{funcs[i], kTierFp64, dims[i], mats[i]};
+  }
   std::vector<int> st(B);
   std::lock_guard<std::mutex> lk(s->mu);
   const int rc = auto_batch(s, reqs, kappa_max, out, kappa, tier_out, st.data());

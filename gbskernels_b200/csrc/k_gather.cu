@@ -90,6 +90,19 @@ __global__ void __launch_bounds__(256) scatter_kernel(ScatterArgs a) {
   }
 }
 
+// Real matrices uploaded as they are, widened to complex on the device (half the bytes to
+// stage and to upload).
+__global__ void expand_real_kernel(const double* __restrict__ in, double2* __restrict__ out, long long n) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = make_double2(in[i], 0.0);
+}
+
+cudaError_t launch_expand_real(const double* in, double* out, long long n, cudaStream_t st) {
+  const int grid = (int)std::min<long long>((n + 255) / 256, 148 * 8);
+  expand_real_kernel<<<grid, 256, 0, st>>>(in, reinterpret_cast<double2*>(out), n);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st) {
   const int total = a.ni + a.ntriv;
   if (total <= 0) return cudaSuccess;

@@ -147,6 +147,13 @@ int gbs_sampler_set_dedup(int on);
  * tier_out[i]: 0 = fp64 value kept, 1 = double-double rerun.                    */
 int gbs_auto_host(int func, const double* mats, int dim, int batch, double kappa_max, double* out,
                   double* kappa, int* tier_out);
+// Uniform batches of real matrices (row-major doubles, dim = matrix side): the results of
+// the complex entry points for the same numbers.  tier: 0 fp64, 1 double-double.
+int gbs_uniform_real_host(int func, int tier, const double* mats, int dim, int batch, double* out);
+int gbs_auto_real_host(int func, const double* mats, int dim, int batch, double kappa_max, double* out,
+                       double* kappa, int* tier_out);
+int gbs_certified_ladder_real_host(int func, const double* mats, int dim, int batch, double rtol, double* out,
+                                   double* bound, int* tier_out);
 
 /* ---- certified tier with the rtol ladder --------------------------------------
  * reference: the certified ladder of gbskernels/__init__.py:374-478 (_certified_single
@@ -221,6 +228,10 @@ int gbs_queue_evaluate_ptrs(gbs_session* s, int batch, const int* funcs, const i
 int gbs_queue_evaluate_auto(gbs_session* s, int batch, const int* funcs, const int* dims, const long long* offsets,
                             const double* mats, double kappa_max, double* out, double* kappa, int* tier_out,
                             int* status);
+// The same with one host pointer per matrix.
+int gbs_queue_evaluate_auto_ptrs(gbs_session* s, int batch, const int* funcs, const int* dims,
+                                 const double* const* mats, double kappa_max, double* out, double* kappa,
+                                 int* tier_out, int* status);
 /* device-resident plan: validate, cut and upload once; run many times on `stream`
  * (a cudaStream_t, or NULL for the session stream); read results back.  Used for
  * timing with inputs resident in HBM and by servers that re-run a fixed batch.   */
