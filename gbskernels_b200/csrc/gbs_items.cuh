@@ -15,7 +15,6 @@
 
 #include "gbs_common.cuh"
 #include "gbs_kernels.cuh"
-#include "haf_dd.cuh"
 #include "haf_pt.cuh"
 #include "haf_rec.cuh"
 #include "perm_tor.cuh"
@@ -107,25 +106,14 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
   ItemResult r{ddc{dd_make(0.0), dd_make(0.0)}, 0.0, kStOk};
   const int N = d.dim, n = N / 2;
   const double* A = mats + d.off;
-  if (TIER == kTierDD) {
-    const HafDDLayout L = haf_dd_layout(haf_smax);
-    ddc acc = ddc{dd_make(0.0), dd_make(0.0)};
-    for (unsigned long long k = 0; k < w.count; ++k) {
-      ddc t = haf_subset_term_dd<false>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane).z;
-      acc = ddc_add(acc, t);
+  if constexpr (TIER == kTierDD || TIER == kTierCertDD) {
+    bool tiny = false;
+    r.val = haf_rec_sum<ddc, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+    if (TIER == kTierCertDD) {
+      const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+      r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj, true);
+      if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
     }
-    r.val = acc;
-  } else if (TIER == kTierCertDD) {
-    // the dd walk and its subset sum, as balls (the value is the dd value bit for bit)
-    const HafDDLayout L = haf_dd_layout(haf_smax, true);
-    ddball acc{ddc{dd_make(0.0), dd_make(0.0)}, 0.0};
-    for (unsigned long long k = 0; k < w.count; ++k) {
-      const ddball t = haf_subset_term_dd<true>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane);
-      acc = ddb_add(acc, t);
-    }
-    r.val = acc.z;
-    r.aux = acc.r;
-    if (!isfinite(acc.r) || !isfinite(acc.z.re.hi) || !isfinite(acc.z.im.hi)) r.st = kStUncertified;
   } else {
     // binary64 tiers: the recursion over pairs (haf_rec.cuh)
     using Z = std::conditional_t<REAL, double, cplx>;
@@ -135,7 +123,7 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
     else r.val = ddc_from_c(v);
     if (TIER == kTierCert) {
       const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
-      r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj);
+      r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj, false);
       // a halving that could round absolutely refuses the certificate
       if (__any_sync(0xffffffffu, tiny)) r.aux = INFINITY;
       if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;

@@ -2,7 +2,6 @@
 // hafnians, one warp per subset, binary64 on the FP64 tensor cores (mma.sync .m16n8k8 /
 // .m16n8k4 .f64).  The cancellation indicator sum |term| of the kappa and auto tiers is
 // defined by these terms; the values come from the recursion over pairs (haf_rec.cuh).
-// The bound path (haf_bound_powers) also serves the certified double-double tier.
 //
 // Algorithm (the reference's, cpu_ref/hafnian.py:101-129 and
 // cpu_ref/loop_hafnian.py:65-108; device form core/hafnian.cu:41-133,
@@ -207,40 +206,6 @@ __device__ __forceinline__ void power_product(const double* __restrict__ P, cons
   }
 }
 
-// Load P (power a, complex, stride ps) into the accumulator layout.
-template <int NT, int MS>
-__device__ __forceinline__ void load_acc(const double* P, int ps, int s, int lane, double (&D)[MS][NT][4]) {
-  const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-  for (int ms = 0; ms < MS; ++ms)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int col = 4 * nt + t4;
-      cplx x0 = mkc(0.0, 0.0), x1 = mkc(0.0, 0.0);
-      if (col < s) {
-        x0 = ld_c(P + ((16 * ms + g) * ps + col) * 2);
-        x1 = ld_c(P + ((16 * ms + g + 8) * ps + col) * 2);
-      }
-      D[ms][nt][0] = x0.re; D[ms][nt][1] = x0.im; D[ms][nt][2] = x1.re; D[ms][nt][3] = x1.im;
-    }
-}
-
-// Store the accumulators into P (rows < 16 MS, columns < s).
-template <int NT, int MS>
-__device__ __forceinline__ void store_acc(double* P, int ps, int s, int lane, const double (&D)[MS][NT][4]) {
-  const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-  for (int ms = 0; ms < MS; ++ms)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int col = 4 * nt + t4;
-      if (col < s) {
-        st_c(P + ((16 * ms + g) * ps + col) * 2, mkc(D[ms][nt][0], D[ms][nt][1]));
-        st_c(P + ((16 * ms + g + 8) * ps + col) * 2, mkc(D[ms][nt][2], D[ms][nt][3]));
-      }
-    }
-}
-
 // ---- one strip of a power in the binary64 value path.  The guards: LIVE (the 8-tile
 // path) keeps every live tile's four columns, including the columns s..4 ntn - 1,
 // which hold zeros wherever they are stored (the staged C, the powers, d); otherwise
@@ -343,98 +308,6 @@ __device__ __forceinline__ void rows_times_d(const double (&D)[1][NT][4], const 
   if (t4 == 0) {
     st_c(Y + (g * hp1 + col) * 2, y0);
     st_c(Y + ((g + 8) * hp1 + col) * 2, y1);
-  }
-}
-
-// ---- bound path helpers (certified tier): real parts only, upward rounding
-template <int NT, int MS>
-__device__ __forceinline__ double even_bound(const double (&D)[MS][NT][4]) {
-  double acc = 0.0;
-#pragma unroll
-  for (int ms = 0; ms < MS; ++ms)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      acc = ru_fma(D[ms][nt][0], shfl_xor_d(D[ms][nt][0], 5), acc);
-      acc = ru_fma(D[ms][nt][2], shfl_xor_d(D[ms][nt][2], 5), acc);
-    }
-  return acc;
-}
-template <int NT, int MS>
-__device__ __forceinline__ double odd_bound(const double (&D)[MS][NT][4], const double* Q, int ps, int s, int lane) {
-  const int g = lane >> 2, t4 = lane & 3;
-  double acc = 0.0;
-#pragma unroll
-  for (int ms = 0; ms < MS; ++ms)
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int col = 4 * nt + t4;
-      if (col < s) {
-        const int cp = col ^ 1;
-        acc = ru_fma(D[ms][nt][0], Q[((16 * ms + (g ^ 1)) * ps + cp) * 2], acc);
-        acc = ru_fma(D[ms][nt][2], Q[((16 * ms + ((g + 8) ^ 1)) * ps + cp) * 2], acc);
-      }
-    }
-  return acc;
-}
-template <int NT, int MS>
-__device__ __forceinline__ void rows_bound(const double (&D)[MS][NT][4], const double* Dv, double* Ym, int col,
-                                           int hp1, int s, int lane) {
-  const int g = lane >> 2, t4 = lane & 3;
-#pragma unroll
-  for (int ms = 0; ms < MS; ++ms) {
-    double y0 = 0.0, y1 = 0.0;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const int c = 4 * nt + t4;
-      if (c < s) {
-        const double dv = ru_abs_c(ld_c(Dv + c * 2));
-        y0 = ru_fma(D[ms][nt][0], dv, y0);
-        y1 = ru_fma(D[ms][nt][2], dv, y1);
-      }
-    }
-#pragma unroll
-    for (int m = 1; m <= 2; m <<= 1) {
-      y0 = ru_add(y0, shfl_xor_d(y0, m));
-      y1 = ru_add(y1, shfl_xor_d(y1, m));
-    }
-    if (t4 == 0) {
-      Ym[(16 * ms + g) * hp1 + col] = y0;
-      Ym[(16 * ms + g + 8) * hp1 + col] = y1;
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Bound path of the certified tiers for the compile-time tile shape: the powers of
-// |C| (Ca; the previous power kept in M) give the trace-bound sums
-// bT[k] += sum_{i,t} M_a[i][t] M_b[i^1][t^1] and the row bounds Ym[row][a] =
-// M_a |d| (upward rounded).  Dv holds d as binary64 complex (zero beyond s).
-template <int NT, int MS>
-__device__ __noinline__ void haf_bound_powers(const double* Ca, double* M, double* Ym, const double* Dv, double* bT,
-                                              int s, int cs, int ps, int n, int h, bool loop, int lane) {
-  const int ntn = (2 * s + 7) >> 3;  // column tiles in use (<= NT)
-  const int hp1 = h + 1;
-  double Dm[MS][NT][4];
-  load_acc<NT, MS>(Ca, cs, s, lane, Dm);
-  {
-    double tb = warp_sum_ru(even_bound<NT, MS>(Dm));
-    if (lane == 0 && 2 <= n) bT[2] = ru_add(bT[2], tb);
-  }
-  if (loop) rows_bound<NT, MS>(Dm, Dv, Ym, 1, hp1, s, lane);
-  for (int a = 2; a <= h; ++a) {
-    const double* Qm = (a == 2) ? Ca : M;
-    const int qs = (a == 2) ? cs : ps;
-    power_product<NT, MS>(Qm, Ca, s, cs, qs, ntn, lane, Dm);
-    double bo = warp_sum_ru(odd_bound<NT, MS>(Dm, Qm, qs, s, lane));
-    double be = warp_sum_ru(even_bound<NT, MS>(Dm));
-    if (lane == 0) {
-      if (2 * a - 1 <= n) bT[2 * a - 1] = ru_add(bT[2 * a - 1], bo);
-      if (2 * a <= n) bT[2 * a] = ru_add(bT[2 * a], be);
-    }
-    __syncwarp();
-    store_acc<NT, MS>(M, ps, s, lane, Dm);
-    if (loop) rows_bound<NT, MS>(Dm, Dv, Ym, a, hp1, s, lane);
-    __syncwarp();
   }
 }
 

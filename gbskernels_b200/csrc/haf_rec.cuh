@@ -1,5 +1,5 @@
-// haf_rec.cuh -- hafnian and loop hafnian by the recursion over pairs, binary64, one
-// warp per block of 2^m0 subsets (m0 <= 7) with every partial state in shared memory.
+// haf_rec.cuh -- hafnian and loop hafnian by the recursion over pairs, binary64 and
+// double-double, one warp per block of 2^m0 subsets (m0 <= 7) with every partial state in shared memory.
 //
 // haf(A) = [z^n] sum_{S subset [n]} (-1)^(n-|S|) f_S(z), the pairs (2u, 2u+1) taken in
 // or left out one after the other (Bjorklund, "Counting perfect matchings as fast as
@@ -41,6 +41,8 @@
 //     are walked breadth-first, so that the small states of up to 16 siblings fill the
 //     32 lanes.
 #pragma once
+
+#include <type_traits>
 
 #include "cert.cuh"
 #include "gbs_common.cuh"
@@ -104,25 +106,34 @@ __host__ __device__ inline HafRecLayout haf_rec_layout(int n, int m0, int L) {
   R.total = o;
   return R;
 }
-// Workspace (doubles) for matrices of side 2n, whatever the split into blocks.
-__host__ __device__ inline int haf_rec_ws(int n, bool loop, bool real) {
+// Workspace (doubles) for matrices of side 2n, whatever the split into blocks; `width`
+// doubles per scalar (1 real, 2 complex, 4 complex double-double).
+__host__ __device__ inline int haf_rec_ws(int n, bool loop, int width) {
   int t = 0;
   for (int m0 = 0; m0 <= n && m0 <= kHafRecBlock; ++m0) {
     const int w = haf_rec_layout(n, m0, loop ? 1 : 0).total;
     t = w > t ? w : t;
   }
-  t = (real ? t : 2 * t) + 2;
-  return (t + 3) & ~3;
+  return (width * t + 5) & ~3;
 }
 
 // ------------------------------------------------------------------ scalars
 template <typename Z> __device__ __forceinline__ Z hz_zero();
 template <> __device__ __forceinline__ cplx hz_zero<cplx>() { return mkc(0.0, 0.0); }
 template <> __device__ __forceinline__ double hz_zero<double>() { return 0.0; }
+template <> __device__ __forceinline__ ddc hz_zero<ddc>() { return ddc{dd_make(0.0), dd_make(0.0)}; }
 __device__ __forceinline__ cplx hz_fma(cplx a, cplx b, cplx c) { return cfma(a, b, c); }
+__device__ __forceinline__ ddc hz_fma(const ddc& a, const ddc& b, const ddc& c) { return ddc_add(c, ddc_mul(a, b)); }
+__device__ __forceinline__ cplx hz_neg(cplx a) { return cneg(a); }
+__device__ __forceinline__ double hz_neg(double a) { return -a; }
+__device__ __forceinline__ ddc hz_neg(const ddc& a) { return ddc_neg(a); }
+__device__ __forceinline__ cplx hz_sum(cplx a) { return warp_sum_c(a); }
+__device__ __forceinline__ double hz_sum(double a) { return warp_sum_d(a); }
+__device__ __forceinline__ ddc hz_sum(const ddc& a) { return warp_sum_ddc(a); }
 __device__ __forceinline__ double hz_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ cplx hz_add(cplx a, cplx b) { return cadd(a, b); }
 __device__ __forceinline__ double hz_add(double a, double b) { return a + b; }
+__device__ __forceinline__ ddc hz_add(const ddc& a, const ddc& b) { return ddc_add(a, b); }
 __device__ __forceinline__ cplx hz_bias(cplx a, double) { return a; }
 __device__ __forceinline__ double hz_bias(double a, double t) { return a + t; }
 template <typename Z> __device__ __forceinline__ Z hz_ld(int i);
@@ -131,7 +142,9 @@ template <> __device__ __forceinline__ cplx hz_ld<cplx>(int i) {
   const double2 v = reinterpret_cast<const double2*>(smem)[i];
   return mkc(v.x, v.y);
 }
+template <> __device__ __forceinline__ ddc hz_ld<ddc>(int i) { return ld_ddc(smem + 4 * i); }
 __device__ __forceinline__ void hz_st(int i, double v) { smem[i] = v; }
+__device__ __forceinline__ void hz_st(int i, const ddc& v) { st_ddc(smem + 4 * i, v); }
 __device__ __forceinline__ void hz_st(int i, cplx v) { reinterpret_cast<double2*>(smem)[i] = make_double2(v.re, v.im); }
 
 // Loads by shared-memory byte address (an address select per load, no branch).
@@ -334,6 +347,56 @@ __device__ __forceinline__ Z haf_rec_e(const HafRecState& s, int m, int c) {
   return x;
 }
 
+// Coefficient c of one output (see HafRecLane): the double-double steps give a lane single
+// coefficients, since a product there is a hundred FP64 instructions against the two loads
+// of its operands, and a whole polynomial would not fit its registers.
+template <typename Z>
+__device__ __forceinline__ Z haf_rec_coef(const HafRecLane& L, int c) {
+  Z x = c <= L.lim ? hz_ld<Z>(L.own + c * L.str) : hz_zero<Z>();
+  const int top = c - 1;
+#pragma unroll 1
+  for (int u = max(0, top - L.limb); u <= min(L.lim, top); ++u)
+    x = hz_fma(hz_ld<Z>(L.a1 + u * L.str), hz_ld<Z>(L.b1 + (top - u) * L.bstr), x);
+#pragma unroll 1
+  for (int u = max(0, top - L.lim2); u <= min(L.lim2, top); ++u)
+    x = hz_fma(hz_ld<Z>(L.a2 + u * L.str), hz_ld<Z>(L.b2 + (top - u) * L.str), x);
+  return x;
+}
+
+// One step: outputs 0 .. cnt - 1 (of(q, active) describes output q), np polynomials and g
+// per state.
+template <typename Z, typename Of>
+__device__ __forceinline__ void haf_rec_step(int T, int cnt, int np, Of of, double bias, int lane) {
+  if constexpr (!std::is_same_v<Z, ddc>) {
+    for (int q0 = 0; q0 < cnt; q0 += 32) haf_rec_dispatch<Z>(T, of(q0 + lane, q0 + lane < cnt), bias);
+  } else {
+    // a lane takes the coefficients h and T + 1 - h of a polynomial: equal work
+    const int H = (T + 3) / 2;
+    for (int x = lane; x < cnt * H; x += 32) {
+      const int q = x / H, h = x - q * H;
+      const HafRecLane L = of(q, true);
+      if (L.a1 == L.own) continue;  // g, below
+      const int h2 = T + 1 - h;
+      hz_st(L.dst + h * L.dstr, haf_rec_coef<Z>(L, h));
+      if (h2 != h) hz_st(L.dst + h2 * L.dstr, haf_rec_coef<Z>(L, h2));
+    }
+    // g: every coefficient reads the lower ones, which a step in place (one state)
+    // overwrites, so they are all formed before any is stored
+    const int states = cnt / (np + 1);
+    for (int x0 = 0; x0 < states * (T + 2); x0 += 32) {
+      const int x = x0 + lane;
+      const bool act = x < states * (T + 2);
+      const int p = act ? x / (T + 2) : 0, c = act ? x - p * (T + 2) : 0;
+      const HafRecLane L = of(p * (np + 1) + np, true);
+      Z v = hz_zero<Z>();
+      if (act) v = haf_rec_coef<Z>(L, c);
+      __syncwarp();
+      if (act) hz_st(L.dst + c * L.dstr, v);
+    }
+  }
+  __syncwarp();
+}
+
 // Take the two highest vertices of state s (m pairs left) into the planes at dst
 // (stride dstr; dst == s.off with dstr == s.str works in place: the rows of the taken
 // vertices lie behind every output).
@@ -345,12 +408,10 @@ __device__ __forceinline__ HafRecState haf_rec_take(const HafRecState& s, const 
     if (lane <= n - m) hz_st(wo + R.e + lane, haf_rec_e<Z>(s, m, lane));
     __syncwarp();
   }
-  for (int q0 = 0; q0 <= np; q0 += 32) {
-    const int q = q0 + lane;
-    const HafRecLane L = haf_rec_lane(s, m, loop, np, q, q <= np, wo + R.zero, wo + R.e, dst, dstr);
-    haf_rec_dispatch<Z>(n - m, L, bias);
-  }
-  __syncwarp();
+  haf_rec_step<Z>(
+      n - m, np + 1, np,
+      [&](int q, bool act) { return haf_rec_lane(s, m, loop, np, q, act, wo + R.zero, wo + R.e, dst, dstr); }, bias,
+      lane);
   return HafRecState{dst, dstr, n - m + 1};
 }
 
@@ -386,31 +447,38 @@ __device__ __forceinline__ Z haf_rec_wide(const HafRecState& root, const HafRecL
       }
       __syncwarp();
     }
-    for (int q0 = 0; q0 < cnt; q0 += 32) {
-      const int qq = q0 + lane;
-      const bool act = qq < cnt;
-      const int p = act ? (int)((unsigned)qq * inv >> 16) : 0;
-      const int q = act ? qq - p * (np + 1) : 0;
-      const HafRecLane L = haf_rec_lane(haf_rec_node(root, R, wo, n, loop, m, p), m, loop, np, q, act, wo + R.zero,
-                                        wo + R.e + p * ec, wo + R.lev[m - 1] + p * dsz, dstr);
-      haf_rec_dispatch<Z>(n - m, L, bias);
-    }
-    __syncwarp();
+    haf_rec_step<Z>(
+        n - m, cnt, np,
+        [&](int qq, bool act) {
+          const int p = act ? (int)((unsigned)qq * inv >> 16) : 0;
+          const int q = act ? qq - p * (np + 1) : 0;
+          return haf_rec_lane(haf_rec_node(root, R, wo, n, loop, m, p), m, loop, np, q, act, wo + R.zero,
+                              wo + R.e + p * ec, wo + R.lev[m - 1] + p * dsz, dstr);
+        },
+        bias, lane);
   }
   Z f = hz_zero<Z>();
-  const int p = lane >> 1, h = lane & 1;
-  {
+  // vertices: haf 0, 1 (b index 0); loop D = 0, then 1, 2 (d: 0 and 1, b: 2)
+  if constexpr (std::is_same_v<Z, ddc>) {
+    // lane: node p, coefficient k of e
+    for (int x = lane; x < (n << (mB - 1)); x += 32) {
+      const int p = x / n, k = x - p * n;
+      const HafRecState s = haf_rec_node(root, R, wo, n, loop, 1, p);
+      const int g = n - 1 - k;
+      if (g > s.lim) continue;
+      const Z e = loop ? haf_rec_e<Z>(s, 1, k) : (k <= s.lim ? hz_ld<Z>(s.off + k * s.str) : hz_zero<Z>());
+      const Z t = ddc_mul(hz_ld<Z>(s.off + s.str - 1 + g * s.str), e);
+      f = ddc_add(f, ((__popc(p) + odd) & 1) ? ddc_neg(t) : t);
+    }
+  } else {
+    const int p = lane >> 1, h = lane & 1;
     const bool act = p < (1 << (mB - 1));
     const HafRecState s = haf_rec_node(root, R, wo, n, loop, 1, act ? p : 0);
     const int g = s.off + s.str - 1;
     const int lim = act ? s.lim : -1;
-    // vertices: haf 0, 1 (b index 0); loop D = 0, then 1, 2 (d: 0 and 1, b: 2)
     f = loop ? haf_rec_f1_dispatch<Z, true>(n - 1, s.off + 2, s.off, s.off + 1, g, s.str, lim, h, wo + R.zero)
              : haf_rec_f1_dispatch<Z, false>(n - 1, s.off, s.off, s.off, g, s.str, lim, h, wo + R.zero);
-    if (!MAJ && ((__popc(p) + odd) & 1)) {
-      if constexpr (sizeof(Z) == sizeof(cplx)) f = cneg(f);
-      else f = -f;
-    }
+    if (!MAJ && ((__popc(p) + odd) & 1)) f = hz_neg(f);
   }
   __syncwarp();
   return f;
@@ -426,6 +494,21 @@ __device__ __forceinline__ void haf_rec_stage(const double* __restrict__ A, int 
   const int V = N + loop, np = V * (V - 1) / 2;
   for (int q = lane; q < np; q += 32) {
     const int j = haf_rec_row(q), k = q - j * (j - 1) / 2;
+    if constexpr (std::is_same_v<Z, ddc>) {
+      // the symmetric part exactly: TwoSum, halved
+      ddc w;
+      if (loop && k == 0) {
+        w = ddc_make(ld_c(A + ((size_t)(j - 1) * N + (j - 1)) * 2));
+      } else {
+        const int r = j - loop, c = k - loop;
+        const cplx x = ld_c(A + ((size_t)r * N + c) * 2), y = ld_c(A + ((size_t)c * N + r) * 2);
+        w.re.hi = two_sum(x.re, y.re, w.re.lo);
+        w.im.hi = two_sum(x.im, y.im, w.im.lo);
+        w = ddc{dd{0.5 * w.re.hi, 0.5 * w.re.lo}, dd{0.5 * w.im.hi, 0.5 * w.im.lo}};
+      }
+      hz_st(off + q, w);
+      continue;
+    }
     cplx w;
     if (loop && k == 0) {
       w = ld_c(A + ((size_t)(j - 1) * N + (j - 1)) * 2);
@@ -438,12 +521,13 @@ __device__ __forceinline__ void haf_rec_stage(const double* __restrict__ A, int 
           fmin(fabs(sum.re) > 0.0 ? fabs(sum.re) : 1.0, fabs(sum.im) > 0.0 ? fabs(sum.im) : 1.0) < 4.450147717014403e-308)
         tiny = true;
     }
-    if constexpr (sizeof(Z) == sizeof(cplx)) hz_st(off + q, w);
-    else hz_st(off + q, MAJ ? ru_abs_c(w) : w.re);
+    if constexpr (std::is_same_v<Z, cplx>) hz_st(off + q, w);
+    if constexpr (std::is_same_v<Z, double>) hz_st(off + q, MAJ ? ru_abs_c(w) : w.re);
   }
   if (lane == 0) {
-    if constexpr (sizeof(Z) == sizeof(cplx)) hz_st(off + np, mkc(1.0, 0.0));
-    else hz_st(off + np, 1.0);
+    if constexpr (std::is_same_v<Z, ddc>) hz_st(off + np, ddc_make(mkc(1.0, 0.0)));
+    if constexpr (std::is_same_v<Z, cplx>) hz_st(off + np, mkc(1.0, 0.0));
+    if constexpr (std::is_same_v<Z, double>) hz_st(off + np, 1.0);
   }
   __syncwarp();
 }
@@ -494,8 +578,7 @@ __device__ __noinline__ Z haf_rec_sum(const double* __restrict__ A, int N, int l
     if (m0 == 0) {  // no pair left: [z^n] g
       Z f = hz_zero<Z>();
       if (lane == 0 && s.lim >= n) f = hz_ld<Z>(wo + n * str0 + g0);
-      if constexpr (sizeof(Z) == sizeof(cplx)) sum = cadd(sum, (!MAJ && (left & 1)) ? cneg(f) : f);
-      else sum += (!MAJ && (left & 1)) ? -f : f;
+      sum = hz_add(sum, (!MAJ && (left & 1)) ? hz_neg(f) : f);
       __syncwarp();
       continue;
     }
@@ -512,12 +595,10 @@ __device__ __noinline__ Z haf_rec_sum(const double* __restrict__ A, int N, int l
         s = r = haf_rec_take<Z>(s, R, wo, n, (d == 2 && t == 2) ? 7 : 6, loop, wo, str0, bias, lane);
       }
       const Z f = haf_rec_wide<Z, MAJ>(r, R, wo, n, loop, (par - __popc(t)) & 1, bias, lane);
-      if constexpr (sizeof(Z) == sizeof(cplx)) sum = cadd(sum, f);
-      else sum += f;
+      sum = hz_add(sum, f);
     }
   }
-  if constexpr (sizeof(Z) == sizeof(cplx)) return warp_sum_c(sum);
-  else return warp_sum_d(sum);
+  return hz_sum(sum);
 }
 
 // ------------------------------------------------------------------ certified radius
@@ -583,12 +664,15 @@ static __device__ const HafRecUnits kHafRecUnits = haf_rec_units_table();
 
 // Radius of the sum over `count` subsets from its majorant sum `maj` (computed to
 // nearest: at most as many roundings, all of positive terms, hence the factor).
-__device__ __forceinline__ double haf_rec_radius(int n, int loop, unsigned count, double maj) {
-  const double blocks = (double)(count >> (count >= (1u << kHafRecBlock) ? kHafRecBlock : 0));
-  const double k = (double)kHafRecUnits.k[loop][n] + 4.0 * blocks + 8.0;  // + the sums over blocks and lanes
+// Double-double: one multiply-add errs by at most 21u^2 |a||v| (product) and 6u^2 of the
+// sum, 28u^2 (|acc| + |a||v|) in all, and its inputs are exact; the same recurrence counts
+// the units.  A lane adds up to 9 terms per breadth-first part there.
+__device__ __forceinline__ double haf_rec_radius(int n, int loop, unsigned count, double maj, bool is_dd) {
+  const double blocks = count >> kHafRecBlock ? (double)(count >> kHafRecBlock) : 1.0;
+  const double k = (double)kHafRecUnits.k[loop][n] + (is_dd ? 40.0 : 4.0) * blocks + 8.0;  // + the sums
   const double g = gamma_ru(k, 3.0 * kU);
   const double up = ru_div(ru_add(maj, 1e-300), rd_sub(1.0, g));
-  return ru_mul(g, up);
+  return ru_mul(is_dd ? gamma_ru(k, 28.0 * kU * kU) : g, up);
 }
 
 }  // namespace gbsb

@@ -27,7 +27,6 @@
 #include <vector>
 
 #include "gbs_kernels.cuh"
-#include "haf_dd.cuh"
 #include "haf_pt.cuh"
 #include "haf_rec.cuh"
 #include "tor_lu.cuh"
@@ -229,9 +228,9 @@ static double item_cost(int fn, int dim, int tier, const Split& S) {
     case kFnTor:
       c = S.param < 0 ? count * dim * dim * dim : count * std::ldexp(120.0, dim / 2 - S.param);
       break;
-    default:  // recursion over pairs; the indicator and the double-double tiers run power traces
+    default:  // recursion over pairs; the indicator tier runs power traces too
       c = count * 12.0 * n * n * (fn == kFnLhaf ? 1.9 : 1.0);
-      if (tier == kTierKappa || is_dd) c += count * (n + 1) * n * n * n;
+      if (tier == kTierKappa) c += count * (n + 1) * n * n * n;
   }
   return is_dd ? 20.0 * c : c;
 }
@@ -263,17 +262,17 @@ static int plan_instance(Plan& P, int fn, int tier, int dim_eval, bool real_in, 
 }
 
 // haf_rec_ws from a table (computed once; a plan asks for every instance).
-static int rec_ws(int n, bool loop, bool real) {
+static int rec_ws(int n, bool loop, int width) {
   struct Table {
-    int w[kHafMaxN / 2 + 1][2][2];
+    int w[kHafMaxN / 2 + 1][2][3];
     Table() {
       for (int i = 0; i <= kHafMaxN / 2; ++i)
         for (int l = 0; l < 2; ++l)
-          for (int r = 0; r < 2; ++r) w[i][l][r] = haf_rec_ws(i, l != 0, r != 0);
+          for (int r = 0; r < 3; ++r) w[i][l][r] = haf_rec_ws(i, l != 0, 1 << r);
     }
   };
   static const Table t;
-  return t.w[n][loop ? 1 : 0][real ? 1 : 0];
+  return t.w[n][loop ? 1 : 0][width >> 1];
 }
 
 static int ws_for_plan(const Plan& P) {
@@ -285,9 +284,9 @@ static int ws_for_plan(const Plan& P) {
     else if (fn == kFnTor && !d.real_in) w = tor_lu_ws_doubles(tier == kTierCert);
     else if (fn == kFnTor)
       w = tor_rec_ws(d.dim / 2, d.param, tier == kTierDD || tier == kTierCertDD, tier_certified(tier));
-    else if (tier == kTierDD || tier == kTierCertDD) w = haf_dd_layout(P.haf_smax, tier == kTierCertDD).total;
     else {
-      w = rec_ws(d.dim / 2, fn == kFnLhaf, d.real_in);
+      const int width = tier == kTierDD || tier == kTierCertDD ? 4 : (d.real_in ? 1 : 2);
+      w = rec_ws(d.dim / 2, fn == kFnLhaf, width);
       if (tier == kTierKappa)  // the power-trace terms use a workspace of the launch's largest side
         w = std::max(w, haf_layout(P.haf_smax).total + (d.real_in ? haf_real_layout(P.haf_smax).total : 0));
     }

@@ -193,7 +193,7 @@ int gbs_haf_noalloc(const double* d_mats, int N, int batch, double* d_out, void*
   L.aux_out = d_aux;
   L.st_out = d_st;
   L.haf_smax = N;
-  L.ws_doubles = haf_rec_ws(n, false, false);
+  L.ws_doubles = haf_rec_ws(n, false, 2);
   constexpr unsigned BR = br1(kFnHaf, kTierFp64);
   const int bps = occ_br<BR>(L, 1);
   int dev = 0, sms = 0;

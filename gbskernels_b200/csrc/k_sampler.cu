@@ -406,7 +406,7 @@ int sampler_chain(const double* h_Ak, long long ak_total, const int* h_off, int 
   L.st_out = B.st.p;
   L.n_items_dev = B.head.p + 1;
   L.haf_smax = slot_max;
-  for (int n = 1; n <= slot_max / 2; ++n) L.ws_doubles = std::max(L.ws_doubles, haf_rec_ws(n, false, false));
+  for (int n = 1; n <= slot_max / 2; ++n) L.ws_doubles = std::max(L.ws_doubles, haf_rec_ws(n, false, 2));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int bps = occ_br<BR>(L, 1);

@@ -106,7 +106,7 @@ extern "C" int t_haf_rec_sum(const double* A, int n, int loop, unsigned lo, int 
   Walk W;
   W.n = n;
   W.loop = loop;
-  if (2 * R.total > haf_rec_ws(n, loop != 0, false)) ++W.bad;
+  if (2 * R.total > haf_rec_ws(n, loop != 0, 2)) ++W.bad;
   auto a = [&](int r, int c) { return Z(A[2 * (r * N + c)], A[2 * (r * N + c) + 1]); };
   const int str0 = haf_rec_polys(m0, loop) + 1;
   Z sum = 0.0;

@@ -1,7 +1,8 @@
 """The hafnian recursion (csrc/haf_rec.cuh) at the sizes and splits where its walk changes:
 no prefix, a prefix, the depth-first part (blocks of 6 and 7 pairs), several blocks per
 item, single-subset items; real and complex, hafnian and loop hafnian, against the
-binary128 oracle; the indicator and certified tiers give the same value."""
+binary128 oracle; the indicator and certified tiers give the same value; the
+double-double tier to its last bit."""
 
 from __future__ import annotations
 
@@ -34,14 +35,18 @@ def test_every_split_vs_oracle(gpu, lib, orc, N):
                 if split > n:
                     continue
                 assert lib.gbs_set_split(code, 0, 2 * n, split, 0) == 0
+                assert lib.gbs_set_split(code, 1, 2 * n, split, 0) == 0
                 try:
                     v = f(A[None])[0]
                     vc, dc = f(A[None], precision="certified", return_diagnostics=True)
                     _, dk = f(A[None], precision="auto", return_diagnostics=True)
+                    vd = f(A[None], precision="dd")[0]
                 finally:
+                    lib.gbs_set_split(code, 1, 2 * n, -1, 0)
                     lib.gbs_set_split(code, 0, 2 * n, -1, 0)
                 assert abs(v - t) <= tol, (func, real, split, v, t)
                 assert vc[0] == v and abs(v - t) <= dc[0]["abs_error_bound"] + U * abs(t), (func, real, split)
+                assert abs(vd - t) <= 2 * U * abs(t) + 1e-20 * absn, (func, real, split, vd, t)
                 assert dk[0]["cancellation"] == pytest.approx(absn / abs(t), rel=1e-6), (func, real, split)
 
 
