@@ -69,10 +69,10 @@ struct HafRecLayout {
   int b5;                            // the state behind (leave, take) of a 7-pair block
   int lev[kHafRecWide];              // lev[m]: states with m pairs left, 2^(mB-1-m) of them
   int zero;                          // one cell that holds zero
-  int e;                             // loop hafnian: the e polynomials of one level
+  int e;                             // loop hafnian: e polynomials (of a step in place; dd: of a level)
   int total;
 };
-__host__ __device__ inline HafRecLayout haf_rec_layout(int n, int m0, int L) {
+__host__ __device__ inline HafRecLayout haf_rec_layout(int n, int m0, int L, bool is_dd = false) {
   HafRecLayout R;
   R.m0 = m0;
   R.mB = m0 < kHafRecWide ? m0 : kHafRecWide;
@@ -96,8 +96,11 @@ __host__ __device__ inline HafRecLayout haf_rec_layout(int n, int m0, int L) {
   R.zero = o++;
   R.e = o;
   if (L) {
-    int es = n;  // one state's e, or those of the 2^(mB-m) nodes of level m
-    for (int m = 2; m <= R.mB; ++m) {
+    // a step out of place keeps e where it will put g' (only the lane that forms g' reads
+    // it, before it writes); the double-double steps, whose lanes take single coefficients
+    // of g', keep those of a whole level
+    int es = n;
+    for (int m = 2; is_dd && m <= R.mB; ++m) {
       const int x = (n - m + 1) << (R.mB - m);
       es = x > es ? x : es;
     }
@@ -111,7 +114,7 @@ __host__ __device__ inline HafRecLayout haf_rec_layout(int n, int m0, int L) {
 __host__ __device__ inline int haf_rec_ws(int n, bool loop, int width) {
   int t = 0;
   for (int m0 = 0; m0 <= n && m0 <= kHafRecBlock; ++m0) {
-    const int w = haf_rec_layout(n, m0, loop ? 1 : 0).total;
+    const int w = haf_rec_layout(n, m0, loop ? 1 : 0, width == 4).total;
     t = w > t ? w : t;
   }
   return (width * t + 5) & ~3;
@@ -297,9 +300,10 @@ struct HafRecState {
 };
 
 // Lane descriptor of output q (a pair index below np, np = g) of a step that takes the
-// two highest vertices of state s with m pairs left.  e: the state's e polynomial (loop).
+// two highest vertices of state s with m pairs left.  e: the state's e polynomial (loop),
+// its coefficients estr apart.
 __host__ __device__ inline HafRecLane haf_rec_lane(const HafRecState& s, int m, int loop, int np, int q, bool active,
-                                                   int zero, int e, int dst, int dstr) {
+                                                   int zero, int e, int estr, int dst, int dstr) {
   HafRecLane L;
   const int V = 2 * m + loop;
   const int r1 = s.off + (V - 1) * (V - 2) / 2, r0 = s.off + (V - 2) * (V - 3) / 2;  // rows of vertices V-1, V-2
@@ -317,7 +321,7 @@ __host__ __device__ inline HafRecLane haf_rec_lane(const HafRecState& s, int m, 
     L.b1 = r1 + V - 2;
     if (loop) {
       L.b1 = e;
-      L.bstr = 1;
+      L.bstr = estr;
       L.limb = kHafMaxN;  // every coefficient up to T
     }
     L.dst = dst + dstr - 1;
@@ -404,13 +408,15 @@ template <typename Z>
 __device__ __forceinline__ HafRecState haf_rec_take(const HafRecState& s, const HafRecLayout& R, int wo, int n, int m,
                                                     int loop, int dst, int dstr, double bias, int lane) {
   const int np = haf_rec_polys(m - 1, loop);
+  const bool own_e = std::is_same_v<Z, ddc> || dst == s.off;
+  const int e = own_e ? wo + R.e : dst + dstr - 1, estr = own_e ? 1 : dstr;
   if (loop) {
-    if (lane <= n - m) hz_st(wo + R.e + lane, haf_rec_e<Z>(s, m, lane));
+    if (lane <= n - m) hz_st(e + lane * estr, haf_rec_e<Z>(s, m, lane));
     __syncwarp();
   }
   haf_rec_step<Z>(
       n - m, np + 1, np,
-      [&](int q, bool act) { return haf_rec_lane(s, m, loop, np, q, act, wo + R.zero, wo + R.e, dst, dstr); }, bias,
+      [&](int q, bool act) { return haf_rec_lane(s, m, loop, np, q, act, wo + R.zero, e, estr, dst, dstr); }, bias,
       lane);
   return HafRecState{dst, dstr, n - m + 1};
 }
@@ -440,10 +446,13 @@ __device__ __forceinline__ Z haf_rec_wide(const HafRecState& root, const HafRecL
     const int dstr = np + 1, dsz = (n - m + 2) * dstr;
     const int ec = n - m + 1;  // coefficients of e
     const unsigned inv = (65536u + np) / (unsigned)(np + 1);  // q / (np + 1) for q < 16 (np + 1), np < 46
+    constexpr bool own_e = std::is_same_v<Z, ddc>;
+    const int eo = own_e ? wo + R.e : wo + R.lev[m - 1] + dstr - 1;  // node 0's e; the next ones epn behind
+    const int epn = own_e ? ec : dsz, estr = own_e ? 1 : dstr;
     if (loop) {
       for (int q = lane; q < (ec << (mB - m)); q += 32) {
-        const int p = q / ec;
-        hz_st(wo + R.e + q, haf_rec_e<Z>(haf_rec_node(root, R, wo, n, loop, m, p), m, q - p * ec));
+        const int p = q / ec, c = q - p * ec;
+        hz_st(eo + p * epn + c * estr, haf_rec_e<Z>(haf_rec_node(root, R, wo, n, loop, m, p), m, c));
       }
       __syncwarp();
     }
@@ -453,7 +462,7 @@ __device__ __forceinline__ Z haf_rec_wide(const HafRecState& root, const HafRecL
           const int p = act ? (int)((unsigned)qq * inv >> 16) : 0;
           const int q = act ? qq - p * (np + 1) : 0;
           return haf_rec_lane(haf_rec_node(root, R, wo, n, loop, m, p), m, loop, np, q, act, wo + R.zero,
-                              wo + R.e + p * ec, wo + R.lev[m - 1] + p * dsz, dstr);
+                              eo + p * epn, estr, wo + R.lev[m - 1] + p * dsz, dstr);
         },
         bias, lane);
   }
@@ -541,7 +550,7 @@ __device__ __noinline__ Z haf_rec_sum(const double* __restrict__ A, int N, int l
   const int n = N / 2;
   const int clog = 31 - __clz(count);
   const int m0 = clog < kHafRecBlock ? clog : kHafRecBlock;
-  const HafRecLayout R = haf_rec_layout(n, m0, loop);
+  const HafRecLayout R = haf_rec_layout(n, m0, loop, std::is_same_v<Z, ddc>);
   const double bias = MAJ ? 0x1p-960 : 0.0;
   const int wo = (int)((ws - smem) / (sizeof(Z) / sizeof(double)));
   const int str0 = haf_rec_polys(m0, loop) + 1;

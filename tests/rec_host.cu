@@ -43,13 +43,13 @@ struct Walk {
     return acc;
   }
   // haf_rec_e of every coefficient
-  void e(const HafRecState& s, int m, int eo) {
+  void e(const HafRecState& s, int m, int eo, int estr) {
     const int V = 2 * m + 1, T = n - m;
     const int r1 = s.off + (V - 1) * (V - 2) / 2, r0 = s.off + (V - 2) * (V - 3) / 2;
     std::vector<Z> x = poly(r1 + V - 2, s.str, s.lim, T), a = poly(r0, s.str, s.lim, T), b = poly(r1, s.str, s.lim, T);
     for (int u = 0; u <= T; ++u)
       for (int v = 0; u + v <= T; ++v) x[u + v] += a[u] * b[v];
-    for (int c = 0; c <= T; ++c) put(eo + c, x[c]);
+    for (int c = 0; c <= T; ++c) put(eo + c * estr, x[c]);
   }
   void lanes(int T, const std::vector<HafRecLane>& ls) {  // 32 lanes at a time: all read, then all write
     for (size_t q0 = 0; q0 < ls.size(); q0 += 32) {
@@ -59,11 +59,13 @@ struct Walk {
         for (int c = 0; c < T + 2; ++c) put(ls[q].dst + c * ls[q].dstr, r[q - q0][c]);
     }
   }
-  HafRecState take(const HafRecState& s, int m, int eo, int dst, int dstr) {
+  HafRecState take(const HafRecState& s, int m, int scratch, int dst, int dstr) {
     const int np = haf_rec_polys(m - 1, loop);
-    if (loop) e(s, m, eo);
+    const bool own_e = dst == s.off;  // in place: e apart, else where g' goes
+    const int eo = own_e ? scratch : dst + dstr - 1, estr = own_e ? 1 : dstr;
+    if (loop) e(s, m, eo, estr);
     std::vector<HafRecLane> ls;
-    for (int q = 0; q <= np; ++q) ls.push_back(haf_rec_lane(s, m, loop, np, q, true, 0, eo, dst, dstr));
+    for (int q = 0; q <= np; ++q) ls.push_back(haf_rec_lane(s, m, loop, np, q, true, 0, eo, estr, dst, dstr));
     lanes(n - m, ls);
     return HafRecState{dst, dstr, n - m + 1};
   }
@@ -72,11 +74,13 @@ struct Walk {
       const int np = haf_rec_polys(m - 1, loop), dstr = np + 1;
       std::vector<HafRecLane> ls;
       if (loop)
-        for (int p = 0; p < (1 << (R.mB - m)); ++p) e(haf_rec_node(root, R, 0, n, loop, m, p), m, R.e + p * (n - m + 1));
+        for (int p = 0; p < (1 << (R.mB - m)); ++p)
+          e(haf_rec_node(root, R, 0, n, loop, m, p), m, R.lev[m - 1] + p * (n - m + 2) * dstr + dstr - 1, dstr);
       for (int p = 0; p < (1 << (R.mB - m)); ++p)
         for (int q = 0; q <= np; ++q)
           ls.push_back(haf_rec_lane(haf_rec_node(root, R, 0, n, loop, m, p), m, loop, np, q, true, 0,
-                                    R.e + p * (n - m + 1), R.lev[m - 1] + p * ((n - m + 2) * dstr), dstr));
+                                    R.lev[m - 1] + p * (n - m + 2) * dstr + dstr - 1, dstr,
+                                    R.lev[m - 1] + p * ((n - m + 2) * dstr), dstr));
       lanes(n - m, ls);
     }
     Z f = 0.0;
