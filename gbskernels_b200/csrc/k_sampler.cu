@@ -171,8 +171,8 @@ __global__ void __launch_bounds__(128) sampler_draw_kernel(const double* __restr
 // prefixes at the last mode against 10^5 draws.  Each prefix is a mixed-radix key
 // (radix cutoff + 1, used only when (cutoff + 1)^(M - 1) < 2^62), inserted into an
 // open-addressing table (linear probing, at least twice as many slots as draws);
-// the occupied slots are numbered by one scan, and every unique prefix is gathered
-// and evaluated once.  A hafnian does not depend on which instance slot holds it,
+// the draw that claims a slot numbers it and is its representative (the numbers come in
+// any order), and every unique prefix is gathered and evaluated once.  A hafnian does not depend on which instance slot holds it,
 // so the draws are bit-identical to evaluating every draw's conditionals.
 constexpr unsigned long long kSamplerEmpty = ~0ull;
 
@@ -186,13 +186,16 @@ __device__ __forceinline__ unsigned long long sampler_mix(unsigned long long x) 
   return x;
 }
 
-// One thread per draw: insert the prefix key; record the draw's table slot and, for
-// the first draw of a key, that draw as the key's representative.  The probe visits
+// One thread per draw: insert the prefix key and record the draw's table slot; the draw
+// that claims a slot takes the next number (*nuniq, zero before) for it: sid[slot], and
+// itself as the representative urep[number].  (A one-block scan numbered the slots before:
+// 230 us a mode for 2^17 of them, half of the chain's GPU time.)  The probe visits
 // each slot at most once (the table has more slots than draws, so it always ends).
 __global__ void __launch_bounds__(128) sampler_key_kernel(const int* __restrict__ state, int M, int d0, int ndraw,
                                                           int k, int radix, unsigned long long* __restrict__ tkeys,
-                                                          int* __restrict__ trep, int tmask,
-                                                          int* __restrict__ slot_of) {
+                                                          int tmask, int* __restrict__ slot_of,
+                                                          int* __restrict__ sid, int* __restrict__ urep,
+                                                          int* __restrict__ nuniq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ndraw) return;
   const int d = d0 + t;
@@ -206,45 +209,15 @@ __global__ void __launch_bounds__(128) sampler_key_kernel(const int* __restrict_
   for (int probe = 0; probe <= tmask; ++probe) {
     const unsigned long long prev = atomicCAS(tkeys + h, kSamplerEmpty, key);
     if (prev == kSamplerEmpty) {
-      trep[h] = d;
+      const int id = atomicAdd(nuniq, 1);
+      sid[h] = id;
+      urep[id] = d;
       break;
     }
     if (prev == key) break;
     h = (h + 1) & (unsigned int)tmask;
   }
   slot_of[t] = (int)h;
-}
-
-// One block: number the occupied slots in slot order (sid[slot], -1 when empty), the
-// representatives urep[id] and the count *nuniq.
-__global__ void __launch_bounds__(kSamplerPlanThreads) sampler_compact_kernel(
-    const unsigned long long* __restrict__ tkeys, const int* __restrict__ trep, int tsize, int* __restrict__ sid,
-    int* __restrict__ urep, int* __restrict__ nuniq) {
-  __shared__ int part[kSamplerPlanThreads];
-  const int tid = threadIdx.x;
-  const int per = (tsize + kSamplerPlanThreads - 1) / kSamplerPlanThreads;
-  const int h0 = min(tsize, tid * per), h1 = min(tsize, h0 + per);
-  int mine = 0;
-  for (int h = h0; h < h1; ++h) mine += tkeys[h] != kSamplerEmpty;
-  part[tid] = mine;
-  __syncthreads();
-  for (int off = 1; off < kSamplerPlanThreads; off <<= 1) {
-    const int v = tid >= off ? part[tid - off] : 0;
-    __syncthreads();
-    part[tid] += v;
-    __syncthreads();
-  }
-  int id = part[tid] - mine;
-  for (int h = h0; h < h1; ++h) {
-    if (tkeys[h] != kSamplerEmpty) {
-      sid[h] = id;
-      urep[id] = trep[h];
-      ++id;
-    } else {
-      sid[h] = -1;
-    }
-  }
-  if (tid == kSamplerPlanThreads - 1) *nuniq = part[tid];
 }
 
 bool g_sampler_dedup = true;  // gbs_sampler_set_dedup
@@ -283,7 +256,7 @@ struct SamplerBufs {
   // prefix deduplication: the table (keys, representative draw, slot number), each
   // draw's slot, the unique prefixes' representatives and their count
   DevBuf<unsigned long long> tkeys;
-  DevBuf<int> trep, sid, slot_of, urep, nuniq;
+  DevBuf<int> sid, slot_of, urep, nuniq;
 };
 constexpr int kSamplerDevs = 64;
 SamplerBufs g_sampler[kSamplerDevs];
@@ -371,7 +344,6 @@ int sampler_chain(const double* h_Ak, long long ak_total, const int* h_off, int 
   int tsize = 1;
   while (tsize < 2 * chunk) tsize <<= 1;
   if (dedup && e == cudaSuccess) e = B.tkeys.need(tsize);
-  if (dedup && e == cudaSuccess) e = B.trep.need(tsize);
   if (dedup && e == cudaSuccess) e = B.sid.need(tsize);
   if (dedup && e == cudaSuccess) e = B.slot_of.need(chunk);
   if (dedup && e == cudaSuccess) e = B.urep.need(chunk);
@@ -406,14 +378,8 @@ int sampler_chain(const double* h_Ak, long long ak_total, const int* h_off, int 
   L.st_out = B.st.p;
   L.n_items_dev = B.head.p + 1;
   L.haf_smax = slot_max;
-  for (int n = 1; n <= slot_max / 2; ++n) L.ws_doubles = std::max(L.ws_doubles, haf_rec_ws(n, false, 2));
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int bps = occ_br<BR>(L, 1);
-  if (bps <= 0) {
-    cudaStreamDestroy(s);
-    return sampler_fail((int)cudaErrorInvalidConfiguration, "sampler: hafnian kernel does not fit");
-  }
   // sampling: modes 1..M; weights only: mode k_stop on the given prefixes
   const int kmax = k_stop > 0 ? k_stop : M;
   const int kfirst = weights_out ? kmax : 1;
@@ -422,15 +388,21 @@ int sampler_chain(const double* h_Ak, long long ak_total, const int* h_off, int 
     const int ni = nd * per;
     for (int k = kfirst; k <= kmax && e == cudaSuccess; ++k) {
       const int slot = std::max(2, std::min(kSamplerMaxN, 2 * k * cutoff));
+      // workspace and blocks for this mode's largest conditional
+      L.ws_doubles = 0;
+      for (int n = 1; n <= slot / 2; ++n) L.ws_doubles = std::max(L.ws_doubles, haf_rec_ws(n, false, 2));
+      const int bps = occ_br<BR>(L, 1);
+      if (bps <= 0) {
+        cudaStreamDestroy(s);
+        return sampler_fail((int)cudaErrorInvalidConfiguration, "sampler: hafnian kernel does not fit");
+      }
       if (dedup) {
         e = cudaMemsetAsync(B.tkeys.p, 0xFF, sizeof(unsigned long long) * tsize, s);
         if (e == cudaSuccess) {
-          sampler_key_kernel<<<(nd + 127) / 128, 128, 0, s>>>(B.state.p, M, d0, nd, k, per, B.tkeys.p, B.trep.p, tsize - 1,
-                                                              B.slot_of.p);
-          e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) {
-          sampler_compact_kernel<<<1, kSamplerPlanThreads, 0, s>>>(B.tkeys.p, B.trep.p, tsize, B.sid.p, B.urep.p, B.nuniq.p);
+          e = cudaMemsetAsync(B.nuniq.p, 0, sizeof(int), s);
+          if (e != cudaSuccess) break;
+          sampler_key_kernel<<<(nd + 127) / 128, 128, 0, s>>>(B.state.p, M, d0, nd, k, per, B.tkeys.p, tsize - 1,
+                                                              B.slot_of.p, B.sid.p, B.urep.p, B.nuniq.p);
           e = cudaGetLastError();
         }
         if (e != cudaSuccess) break;
