@@ -26,8 +26,8 @@
 //     2^kTail subsets by a compile-time recursion, the last mode by its 2 x 2 determinant.
 // Bound by latency and the issue of its instruction stream (about 3,700 warp instructions
 // per 512 subsets, a quarter of them FP64), not by the FP64 pipe.  Measured, against one
-// 10 x 10 factorisation per lane and subset: 64 x 20 modes 5.98 -> 1.60 ms, 512 x 12 modes
-// 0.340 -> 0.113 ms.
+// 10 x 10 factorisation per lane and subset: 64 x 20 modes 5.98 -> 1.43 ms, 512 x 12 modes
+// 0.340 -> 0.091 ms.
 //
 // Certified tiers: see tor_warp.cuh (the a-posteriori radius |t| rho_m of a term of
 // dimension m); the step above satisfies its premises: every factor entry is an inner
@@ -296,7 +296,8 @@ __device__ __forceinline__ void ts_ld_pair(const double* ws, int i, dd& a, dd& b
 
 // The breadth-first levels M .. tail + 1 of a full walk (root w at mW = tail + 5), every
 // size a constant and the entries from the map: index arithmetic on runtime sizes was half
-// of the walk's instructions (16 modes, 512 instances: 838 us before).
+// of the walk's instructions (16 modes, 512 instances: 838 us before, 704 with the entry
+// loops unrolled whole).
 template <typename S, int M>
 __device__ __forceinline__ void tor_rec_levels(double* ws, const TorRecLayout& R, const TorRecState& w, int lane,
                                                bool& ok) {
@@ -321,7 +322,7 @@ __device__ __forceinline__ void tor_rec_levels(double* ws, const TorRecLayout& R
 #pragma unroll
     for (int q0 = 0; q0 < N * rows; q0 += 32) {
       const int q = q0 + lane;
-      if (q < N * rows) {
+      if (q0 + 32 <= N * rows || q < N * rows) {
         const int p = q / rows, j = q - p * rows;
         const int o = noff[p], v = R.piv + 3 * p;
         const S l0 = ts_mul(ts_ld(ws, o + ra + j, z), ts_ld(ws, v, z));
@@ -334,11 +335,11 @@ __device__ __forceinline__ void tor_rec_levels(double* ws, const TorRecLayout& R
     constexpr int mo = tor_rec_map_off(TAIL, M);
     const int dst = R.lev + mo;
     // double-word steps are thirty times as long: unrolled they only miss the instruction cache
-    constexpr int UN = TorRec<S>::W == 1 ? 6 : 1;
+    constexpr int UN = TorRec<S>::W == 1 ? 32 : 1;
 #pragma unroll UN
     for (int q0 = 0; q0 < N * E; q0 += 32) {
       const int q = q0 + lane;
-      if (q < N * E) {
+      if (q0 + 32 <= N * E || q < N * E) {
         const unsigned x = tor_rec_map<TAIL>(mo + q);
         const int p = (int)(x >> 24);
         S l0i, l1i, l0j, l1j;
@@ -419,7 +420,7 @@ __device__ __forceinline__ TorRecSum<S, AUX> tor_rec_tail_load(const double* ws,
 // positive.
 template <typename S, int AUX>
 static __device__ __noinline__ bool tor_rec_item(const double* __restrict__ Oc, int k, int g, uint32_t pat, double* ws,
-                                                 const TorRecLayout& R, const double* rho, int lane, S& total,
+                                                 const TorRecLayout R, const double* rho, int lane, S& total,
                                                  double& aux) {
   constexpr int TAIL = TorRec<S>::kTail;
   const S z{};
