@@ -12,8 +12,8 @@ weights gamma ~ CN(0, 0.1) on the loop-hafnian diagonals (gbskernels_b200.worklo
   e2e      the same through the public API (Workspace.evaluate) from host numpy
            buffers, H2D of the matrices and D2H of the results inside the timed region
   plain_per_size  the same batch as one launch per (function, size) bucket
-  roofline reference-algorithm FP64 flops of the batch / kernel time, against the
-           FP64 tensor-core peak measured live by gbs_probe_fp64_peak
+  roofline FP64 flops of the batch by the algorithm in use (workloads.walk_flops) /
+           kernel time, against the FP64 peak measured live by gbs_probe_fp64_peak
   cpu_baseline    the oracle (binary64 restatement of the reference algorithm) on the
            host cores, stratified sample: three haf + three lhaf instances per size class
   plain_per_size_sync  the reference's plain per-size path (gbskernels/__init__.py:
@@ -377,18 +377,16 @@ def other_configs(G, peak, cores):
     session's CUDA events; warm-up run first), with parity spot checks."""
     from gbskernels_b200 import configs, workloads
     out = {}
-    flops = workloads.ref_flops
+    flops = workloads.walk_flops
     jobs = []
     # config 1: 4096 real symmetric 16 x 16 hafnians
     c1 = list(workloads.haf_real_batch(4096, 16, seed=1))
-    f1 = 4096 * flops("haf", 16)              # the reference evaluates real input as complex
-    f1r = 4096 * flops("haf", 16, real=True)  # the same walk in real arithmetic
+    f1 = 4096 * flops("haf", 16, real=True)
     r, v, a, st = configs.run("haf", c1, "fp64", reps=3)
     rc, vc, ac, stc = configs.run("haf", c1, "certified", reps=2)
     out["config1_haf16_real"] = {
         "batch": 4096, "value": r["instances_per_s"], "unit": "instances/s", "kernel_ms": r["kernel_ms"],
         "roofline_frac": f1 / (r["kernel_ms"] * 1e-3) / 1e12 / peak,
-        "roofline_frac_real_flops": f1r / (r["kernel_ms"] * 1e-3) / 1e12 / peak,
         "certified": {"value": rc["instances_per_s"], "rel_bound_median": rc["rel_bound_median"],
                       "values_equal_fp64": bool(np.array_equal(vc, v))}}
     jobs += [("c1", i, "haf", c1[i].astype(np.complex128), v[i], ac[i]) for i in range(4)]
@@ -464,7 +462,8 @@ def main():
     tiers = np.zeros(B, dtype=np.int32)
     buf, dims, offs = G._pack(mats)
     in_bytes = buf.nbytes
-    algo_flops = float(sum(workloads.ref_flops(f, m.shape[0]) for f, m in zip(funcs, mats)))
+    algo_flops = float(sum(workloads.walk_flops(f, m.shape[0]) for f, m in zip(funcs, mats)))
+    ref_flops = float(sum(workloads.ref_flops(f, m.shape[0]) for f, m in zip(funcs, mats)))
 
     ws = G.Workspace()
     ws.__enter__()
@@ -535,19 +534,16 @@ def main():
                                    f"photon-pattern submatrices, gamma ~ CN(0,0.1)",
                        "batch": B, "parallelism": f"replicas x{dist.world}",
                        "l2": f"inputs {in_bytes / 1e6:.0f} MB per rank > 126 MB L2 (no flush needed)"},
-            "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
-                         # DRAM read + write bytes of one launch: an ncu capture of this
-                         # kernel on the 256-instance case (--profile-small) read 1.741568 MB
-                         # and wrote 0 B; scaled by the instances per launch (each matrix is
-                         # read once, so DRAM traffic grows in proportion)
-                         "traffic": 1.741568e6 / 256 * B,
-                         "traffic_unit": "bytes per launch (ncu capture scaled by instances)",
-                         "peak_source": "FP64 mma.m16n8k8 throughput measured live (gbs_probe_fp64_peak); "
-                                        "MEASURED_PEAKS.json has no FP64 figure",
-                         "flops_per_step": algo_flops,
-                         "flops_note": "reference-algorithm flops (n-1 power products per subset); the "
-                                       "kernel executes ceil(n/2)-1 products per subset"},
+                         # each matrix is read once and each value written once
+                         "traffic": in_bytes + 28 * B,
+                         "traffic_unit": "bytes per launch (inputs and results, not measured)",
+                         "peak_source": "FP64 mma.m16n8k8 throughput measured live (gbs_probe_fp64_peak), the "
+                                        "same as the FMA pipe's; MEASURED_PEAKS.json has no FP64 figure",
+                         "flops_per_step": algo_flops, "reference_flops_per_step": ref_flops,
+                         "flops_note": "flops of the recursion over pairs; the reference's power trace would "
+                                       "take reference_flops_per_step"},
             "clocks": clk, "gpu_launches": launches_per_step * a.steps, "check": check}
 
     if a.profile_small:

@@ -10,7 +10,7 @@ reference's CPU backend (``backend="cpu"``) and its mpmath tier (``"ref"``) stay
 in the reference package.
 
 Precision tiers (as in the reference):
-  * ``"fp64"``      binary64 throughout (power trace products on FP64 tensor cores);
+  * ``"fp64"``      binary64 throughout;
   * ``"dd"``        double-double value path;
   * ``"auto"``      fp64 plus the cancellation indicator kappa = sum|term| / |value|,
                     elements with kappa >= 1e8 rerun in double-double ON THE DEVICE

@@ -208,3 +208,22 @@ def ref_flops(func: str, dim: int, real: bool = False) -> float:
         k = dim // 2
         return 2.0 * 2.0 ** k * (k * k - k + 1)
     raise ValueError(func)
+
+
+def walk_flops(func: str, dim: int, real: bool = False) -> float:
+    """FP64 flops of this library's own algorithm for one instance (complex multiply-add =
+    8, real = 2): the recursion over pairs for haf / lhaf (csrc/haf_rec.cuh), the recursion
+    over modes for tor (csrc/tor_rec.cuh), the Glynn walk for perm."""
+    if func in ("haf", "lhaf"):
+        n = (dim + 1) // 2
+        loop = func == "lhaf"
+        macs = 0.0
+        for m in range(1, n + 1):
+            t = n - m  # 2^t states of m pairs, polynomials of t + 1 coefficients
+            polys = (m - 1) * (2 * m - 3 + (2 if loop else 0))
+            macs += 2.0 ** t * (polys * (t + 1) * (t + 2) + (t + 1) * (t + 2) / 2 * (2 if loop else 1))
+        return macs * (2.0 if real else 8.0)
+    if func == "tor":
+        k = dim // 2
+        return sum(2.0 ** (k - m - 1) * (4.0 * m * (2 * m + 1) + 20.0) for m in range(k))
+    return ref_flops(func, dim, real)
