@@ -66,8 +66,9 @@ def _as_stack(matrices: Iterable[Any]) -> np.ndarray:
     takes it as it is), complex128 otherwise."""
     arr = np.asarray(matrices)
     real = arr.dtype.kind in "fiub" and arr.dtype.itemsize <= 8
-    stack = np.ascontiguousarray(arr if real else np.asarray(matrices, dtype=np.complex128),
-                                 dtype=np.float64 if real else np.complex128)
+    if not real and arr.dtype.kind not in "cf":  # objects, texts: numpy's own conversion of the input
+        arr = np.asarray(matrices, dtype=np.complex128)
+    stack = np.ascontiguousarray(arr, dtype=np.float64 if real else np.complex128)
     if stack.ndim != 3 or stack.shape[1] != stack.shape[2]:
         raise ValueError(
             "GPU backend needs a uniform (B, d, d) stack of square matrices; "
