@@ -701,8 +701,8 @@ class Workspace:
 
     def _call_ptrs(self, funcs, mats, precisions, out, aux, st) -> None:
         ptr, dims, keep = _pointers(mats)
-        fns = np.fromiter(map(_FN.__getitem__, funcs), dtype=np.int32, count=len(funcs))
-        tiers = np.fromiter(map(_TIER.__getitem__, precisions), dtype=np.int32, count=len(precisions))
+        fns = np.fromiter(map(_FN.__getitem__, funcs), dtype=np.int32)
+        tiers = np.fromiter(map(_TIER.__getitem__, precisions), dtype=np.int32)
         rc = _lib.load().gbs_queue_evaluate_ptrs(
             self._session, len(mats), _lib.iptr(fns), _lib.iptr(tiers), _lib.iptr(dims),
             ctypes.c_void_p(ptr.ctypes.data), 0 if self._persistent else 1,

@@ -58,3 +58,25 @@ def test_a_mixed_list_is_complex(G):
 def test_refused_batches(G, batch):
     with pytest.raises((ValueError, TypeError)):
         G._as_stack(batch)
+
+
+class _Recorder:
+    """A library whose queue call notes the function and tier codes it gets."""
+
+    def gbs_queue_evaluate_ptrs(self, session, B, fns, tiers, dims, *rest):
+        self.codes = [fns[i] for i in range(B)], [tiers[i] for i in range(B)], [dims[i] for i in range(B)]
+        return 0
+
+
+@pytest.mark.parametrize("wrap", [list, tuple, iter, lambda x: (y for y in x), lambda x: map(str, x),
+                                  lambda x: np.array(x), lambda x: dict(enumerate(x)).values()])
+def test_names_of_a_mixed_batch_may_be_any_iterable(G, monkeypatch, wrap):
+    rec = _Recorder()
+    monkeypatch.setattr(G._lib, "load", lambda: rec)
+    ws = G.Workspace()
+    ws._session = object()
+    mats = [np.eye(n, dtype=complex) for n in (2, 4, 6)]
+    for call in (ws.evaluate, ws.evaluate_full):
+        call(wrap(["haf", "lhaf", "tor"]), mats, wrap(["fp64", "dd", "fp64"]))
+        assert rec.codes == ([1, 2, 3], [0, 1, 0], [2, 4, 6])
+    ws._session = None
