@@ -110,8 +110,11 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
     bool tiny = false;
     r.val = haf_rec_sum<ddc, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
     if (TIER == kTierCertDD) {
-      const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+      // the majorant's own halvings are those of the high words: exact if `tiny` is clear
+      bool high = false;
+      const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, high);
       r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj, true);
+      if (__any_sync(0xffffffffu, tiny)) r.aux = INFINITY;
       if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
     }
   } else {

@@ -496,7 +496,10 @@ __device__ __forceinline__ Z haf_rec_wide(const HafRecState& root, const HafRecL
 // Stage the root: the symmetric part (A + A^T) / 2 (exact for a symmetric A; the sum
 // over perfect matchings does not see the antisymmetric part to first order), or an
 // upper bound of its modulus (MAJ); loop weights A_vv as they are.  `tiny`: a halving
-// that could round absolutely (certified tier).
+// that could round absolutely (certified tiers: no radius relative to the entries covers
+// that).  Binary64: a sum of unequal entries below twice the smallest normal number.
+// Double-double: halves that do not double back, in either word -- the low one can be
+// subnormal where the high one is normal.
 template <typename Z, bool MAJ>
 __device__ __forceinline__ void haf_rec_stage(const double* __restrict__ A, int N, int loop, int off, int lane,
                                               bool& tiny) {
@@ -511,9 +514,10 @@ __device__ __forceinline__ void haf_rec_stage(const double* __restrict__ A, int 
       } else {
         const int r = j - loop, c = k - loop;
         const cplx x = ld_c(A + ((size_t)r * N + c) * 2), y = ld_c(A + ((size_t)c * N + r) * 2);
-        w.re.hi = two_sum(x.re, y.re, w.re.lo);
-        w.im.hi = two_sum(x.im, y.im, w.im.lo);
-        w = ddc{dd{0.5 * w.re.hi, 0.5 * w.re.lo}, dd{0.5 * w.im.hi, 0.5 * w.im.lo}};
+        double er, ei;
+        const double sr = two_sum(x.re, y.re, er), si = two_sum(x.im, y.im, ei);
+        w = ddc{dd{0.5 * sr, 0.5 * er}, dd{0.5 * si, 0.5 * ei}};
+        if (2.0 * w.re.hi != sr || 2.0 * w.re.lo != er || 2.0 * w.im.hi != si || 2.0 * w.im.lo != ei) tiny = true;
       }
       hz_st(off + q, w);
       continue;
