@@ -44,8 +44,12 @@ namespace gbsb {
 constexpr int kTorRecWide = 5;  // modes walked breadth-first
 
 template <typename S> struct TorRec;
-template <> struct TorRec<double> { static constexpr int kTail = 4; static constexpr int W = 1; };
-template <> struct TorRec<dd> { static constexpr int kTail = 3; static constexpr int W = 2; };
+template <> struct TorRec<double> {
+  static constexpr int kTail = 4, W = 1, kOrder = 5;  // modes per lane, doubles per scalar, tor_rec_source's tail
+};
+template <> struct TorRec<dd> {
+  static constexpr int kTail = 3, W = 2, kOrder = 4;
+};
 
 // Row i of packed entry e = i (i + 1) / 2 + j, i < 64 (32 modes).
 struct TorRecTri {
@@ -199,6 +203,17 @@ __device__ __forceinline__ dd ts_ld(const double* ws, int i, dd) { return ld_dd(
 __device__ __forceinline__ void ts_st(double* ws, int i, double v) { ws[i] = v; }
 __device__ __forceinline__ void ts_st(double* ws, int i, dd v) { st_dd(ws + 2 * i, v); }
 __device__ __forceinline__ double ts_fms(double a, double b, double c) { return fma(-b, c, a); }
+// The entry of O read for row i, column j <= i of M.  O is meant to be symmetric; of one that
+// is not, the torontonian reads the lower triangle in the order (mode, x before p), as the
+// reference does, but for the block of the last `tail` modes (5, double-double 4) against the
+// modes before them, where it reads the upper one.
+__host__ __device__ inline void tor_rec_source(int k, int tail, int i, int j, int& row, int& col) {
+  const int mi = k - 1 - (i >> 1), mj = k - 1 - (j >> 1);  // modes, mi <= mj
+  const int a = mi + (i & 1) * k, b = mj + (j & 1) * k;
+  const bool upper = mi == mj || (mi < k - tail && mj >= k - tail);
+  row = upper ? a : b;
+  col = upper ? b : a;
+}
 __device__ __forceinline__ dd ts_fms(dd a, dd b, dd c) { return dd_fms(a, b, c); }
 __device__ __forceinline__ double ts_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ dd ts_mul(dd a, dd b) { return dd_mul(a, b); }
@@ -425,10 +440,11 @@ static __device__ __noinline__ bool tor_rec_item(const double* __restrict__ Oc, 
   constexpr int TAIL = TorRec<S>::kTail;
   const S z{};
   const int dim = 2 * k;
-  auto comp = [&](int r) { return (k - 1 - (r >> 1)) + (r & 1) * k; };  // row -> component of O
   for (int e = lane; e < tor_rec_entries(k); e += 32) {
     const int i = tor_rec_row(e), j = e - i * (i + 1) / 2;
-    ts_st(ws, e, ts_m(Oc, dim, comp(i), comp(j), z));
+    int r, c;
+    tor_rec_source(k, TorRec<S>::kOrder, i, j, r, c);
+    ts_st(ws, e, ts_m(Oc, dim, r, c, z));
   }
   if (lane == 0) ts_st(ws, R.t, ts_make(1.0, z));
   __syncwarp();

@@ -72,3 +72,14 @@ def test_accesses_stay_inside_the_workspace(torlib, k):
                     _item(torlib, O, g, lo, is_dd, cert)
     if k <= 17:
         _item(torlib, O, 0, 0, 0, 1)  # more free modes than are walked at a time
+
+
+@pytest.mark.parametrize("k", [2, 5, 6, 9])
+def test_an_asymmetric_O_reads_one_entry_of_each_pair(torlib, orc, k):
+    from test_gpu_tor_order import asymmetric_O, entries_read
+    O = asymmetric_O(k, k)
+    for is_dd, tail in ((0, 5), (1, 4)):
+        v = _item(torlib, O, 0, 0, is_dd, 0)
+        assert v == _item(torlib, entries_read(O, tail), 0, 0, is_dd, 0)
+        if k <= tail:
+            assert v == pytest.approx(orc.tor(O.astype(complex)).real, rel=1e-10)

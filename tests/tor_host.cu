@@ -103,9 +103,10 @@ extern "C" int t_tor_rec_item(const double* O, int k, int g, unsigned lo, int is
     const int g2 = k - f;
     x.w.assign(R.rho, 0.0);
     x.set.assign(R.rho, 0);
-    auto comp = [&](int r) { return (k - 1 - (r >> 1)) + (r & 1) * k; };
     for (int e = 0; e < tor_rec_entries(k); ++e) {
-      const int i = tor_rec_row(e), j = e - i * (i + 1) / 2, a = comp(i), b = comp(j);
+      const int i = tor_rec_row(e), j = e - i * (i + 1) / 2;
+      int a, b;
+      tor_rec_source(k, is_dd ? TorRec<dd>::kOrder : TorRec<double>::kOrder, i, j, a, b);
       x.put(e, (a == b ? 1.0 : 0.0) - O[a * dim + b]);
     }
     x.put(R.t, 1.0);
