@@ -122,7 +122,8 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
     using Z = std::conditional_t<REAL, double, cplx>;
     bool tiny = false;
     const Z v = haf_rec_sum<Z, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
-    if constexpr (REAL) r.val = ddc{dd_make(v), dd_make(0.0)};
+    // a real value that is not finite is NaN in both parts, as in complex arithmetic
+    if constexpr (REAL) r.val = ddc_from_c(isfinite(v) ? mkc(v, 0.0) : mkc(NAN, NAN));
     else r.val = ddc_from_c(v);
     if (TIER == kTierCert) {
       const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
