@@ -150,19 +150,20 @@ __device__ __forceinline__ void hz_st(int i, double v) { smem[i] = v; }
 __device__ __forceinline__ void hz_st(int i, const ddc& v) { st_ddc(smem + 4 * i, v); }
 __device__ __forceinline__ void hz_st(int i, cplx v) { reinterpret_cast<double2*>(smem)[i] = make_double2(v.re, v.im); }
 
-// Loads by shared-memory byte address (an address select per load, no branch).
+// Loads by shared-memory byte address (an address select per load, no branch).  They read
+// what hz_st wrote, so the compiler is told that they read memory.
 __device__ __forceinline__ uint32_t hz_addr(int i, int bytes) {
   return (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)(i * bytes);
 }
 template <typename Z> __device__ __forceinline__ Z hz_lds(uint32_t a);
 template <> __device__ __forceinline__ double hz_lds<double>(uint32_t a) {
   double x;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a));
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a) : "memory");
   return x;
 }
 template <> __device__ __forceinline__ cplx hz_lds<cplx>(uint32_t a) {
   cplx x;
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.re), "=d"(x.im) : "r"(a));
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.re), "=d"(x.im) : "r"(a) : "memory");
   return x;
 }
 
@@ -236,8 +237,10 @@ __device__ __noinline__ Z haf_rec_f1(int b, int d0, int d1, int g, int str, int 
     }
 #pragma unroll
     for (int c = 0; c <= T; ++c) {
+      // of the odd half acc[T] lies beyond z^(n-1), perhaps beyond the number range: left out,
+      // not multiplied by zero
       const int k = T - h - c;
-      f = hz_fma(acc[c], hz_ld<Z>(k >= 0 && k <= lim ? g + k * str : zero), f);
+      f = hz_fma(c < T || k == 0 ? acc[c] : hz_zero<Z>(), hz_ld<Z>(k >= 0 && k <= lim ? g + k * str : zero), f);
     }
   }
 #pragma unroll

@@ -52,3 +52,25 @@ def test_an_entry_that_is_not_finite(gpu, func, n, real):
                 assert np.isnan(v[1:-1].imag).all(), (precision, v)
         with pytest.raises((RuntimeError, ValueError), match="finite input"):
             f(bad, precision="certified", return_diagnostics=True)
+
+
+@pytest.mark.parametrize("func,n,real", [c for c in CASES if c[0] != "tor" and c[1] % 2 == 0])
+def test_powers_of_two(gpu, func, n, real):
+    f = getattr(gpu, f"{func}_batched")
+    A = _mat(func, n, real)
+    one = {p: f(A[None], precision=p)[0] for p in ("fp64", "dd")}
+    # every edge times 2^e, every loop times 2^(e / 2): the value times 2^(e n / 2).  Double
+    # words need their low parts above 2^-1022, entries their products below 2^1024.
+    for e in {2 * (400 // n), -2 * (400 // n), 2 * (900 // n), 2 * (9000 // n)}:
+        S = A * 2.0 ** min(e, 1000)
+        if func == "lhaf":
+            S[np.arange(n), np.arange(n)] = np.diag(A) * 2.0 ** (min(e, 1000) // 2)
+        for p in ("fp64", "dd"):
+            v = f(S[None], precision=p)[0]
+            if e * n // 2 < 1000:
+                assert v == one[p] * 2.0 ** (e * n // 2), (p, e)
+            elif n > 2:
+                assert np.isnan(v.real) and np.isnan(v.imag), (p, e, v)
+    if n > 2:
+        with pytest.raises(FloatingPointError):
+            f(A[None] * 2.0 ** 1000, precision="certified", return_diagnostics=True)
