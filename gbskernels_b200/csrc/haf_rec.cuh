@@ -150,20 +150,19 @@ __device__ __forceinline__ void hz_st(int i, double v) { smem[i] = v; }
 __device__ __forceinline__ void hz_st(int i, const ddc& v) { st_ddc(smem + 4 * i, v); }
 __device__ __forceinline__ void hz_st(int i, cplx v) { reinterpret_cast<double2*>(smem)[i] = make_double2(v.re, v.im); }
 
-// Loads by shared-memory byte address (an address select per load, no branch).  They read
-// what hz_st wrote, so the compiler is told that they read memory.
+// Loads by shared-memory byte address (an address select per load, no branch).
 __device__ __forceinline__ uint32_t hz_addr(int i, int bytes) {
   return (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)(i * bytes);
 }
 template <typename Z> __device__ __forceinline__ Z hz_lds(uint32_t a);
 template <> __device__ __forceinline__ double hz_lds<double>(uint32_t a) {
   double x;
-  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a) : "memory");
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(a));
   return x;
 }
 template <> __device__ __forceinline__ cplx hz_lds<cplx>(uint32_t a) {
   cplx x;
-  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.re), "=d"(x.im) : "r"(a) : "memory");
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.re), "=d"(x.im) : "r"(a));
   return x;
 }
 
