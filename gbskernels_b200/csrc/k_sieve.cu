@@ -58,7 +58,10 @@ namespace gbsb {
 constexpr int kSieveMaxM = 32;
 constexpr int kSieveMaxN = 64;
 constexpr int kSieveMaxK = kSieveMaxN / 2;
-constexpr long long kSieveMaxItems = 1ll << 26;  // partial storage: 1 GiB
+// Size limit of a call, counted in items of 256 terms (longer ones for a pattern of more than
+// 2^28).  The walk's own items (16 bytes of partial sum each, certified 24) are at most twice
+// as many, but for patterns of fewer than 14,560 terms: at most 65 each, of 32 terms or more.
+constexpr long long kSieveMaxItems = 1ll << 26;
 
 struct SievePattern {
   unsigned long long terms;  // sieve terms walked (top digit halved)
@@ -76,7 +79,7 @@ struct SievePattern {
 };
 
 constexpr int kSieveLowDigits = 5;    // 2^5 = 32 combinations at least, when there are as many
-constexpr int kSieveLowTerms = 512;
+constexpr int kSieveLowTerms = 512;   // room for the last digit added: 31 combinations times up to 16 values
 constexpr int kSieveWarps = 4;
 
 // Per-warp tables of an item.
@@ -474,9 +477,9 @@ int sieve_run(const double* A_in, const double* gamma, int M, const int* reps, i
            P.plow * P.radix[P.nlow] <= kSieveLowTerms &&
            P.terms / (unsigned long long)(P.plow * P.radix[P.nlow]) >= 32)
       P.plow *= P.radix[P.nlow++];
-    // an item is one group of 32 lanes' walks, more for a long pattern (at most 2^20 items)
-    // (and 256 terms at least in a huge batch, which bounds the partials)
-    P.groups = batch >= (1 << 16) ? std::max(1, 8 / P.plow) : 1;
+    // an item is one group of 32 lanes' walks, more for a long pattern (at most 2^20 items):
+    // a function of the pattern alone, so that its sum does not depend on the batch
+    P.groups = 1;
     while (P.terms > 32ull * P.plow * P.groups * (1ull << 20)) P.groups <<= 1;
     P.item_len = 32ull * P.plow * P.groups;
     P.item0 = items;

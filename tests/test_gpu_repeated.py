@@ -177,3 +177,14 @@ def test_batch_equals_single_bitwise(gpu):
     got = gpu.lhaf_repeated(A, g, reps)
     for b in range(6):
         assert gpu.lhaf_repeated(A, g, reps[b]) == got[b]
+
+
+def test_huge_batch_equals_single_bitwise(gpu):
+    # a pattern's sum is grouped the same way in a batch of 2^16 and alone, where few
+    # combinations are walked by a lane and the others take several groups of 32 lanes
+    for pats in ([[2, 40], [20, 20], [30, 33], [1, 60], [40, 4]], [[4, 6, 8], [2, 6, 20], [5, 5, 9], [1, 1, 40], [6, 8, 9]]):
+        pats = np.array(pats, np.int32)
+        A, g = base(pats.shape[1])
+        alone = np.array([gpu.lhaf_repeated(A, g, p) for p in pats])
+        batch = gpu.lhaf_repeated(A, g, np.tile(pats, ((1 << 16) // len(pats) + 1, 1)))
+        assert np.array_equal(batch, np.tile(alone, len(batch) // len(alone)))
