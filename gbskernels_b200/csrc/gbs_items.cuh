@@ -205,10 +205,8 @@ __device__ ItemResult tor_item(const double* __restrict__ mats, const InstDesc& 
   double aux = 0.0;
   bool ok = true;
   if (proved) {
-    const unsigned long long subs = 1ull << (n - f - d.param);
-    for (unsigned long long p = 0; p < w.count * subs; ++p) {
-      // pattern over the first n - f modes: the item's own bits lowest
-      const uint32_t pat = (uint32_t)((w.lo + p / subs) | ((p % subs) << d.param));
+    for (unsigned long long p = 0; p < (unsigned long long)w.count << (n - f - d.param); ++p) {
+      const uint32_t pat = tor_rec_pattern(w.lo, p, d.param, n - f);
       S t = ts_make(0.0, S{});
       double a = 0.0;
       ok = tor_rec_item<S, AUX>(Oc, n, n - f, pat, ws, R, rho, lane, t, a) && ok;

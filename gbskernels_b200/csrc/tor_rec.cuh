@@ -129,6 +129,12 @@ __host__ __device__ inline int tor_rec_lev(const TorRecLayout& R, int m, int slo
 // SM instead of 7, but stages the matrix four times as often: 20 modes 1.89 against 1.60 ms.
 constexpr int kTorRecFree = 14;
 __host__ __device__ inline int tor_rec_free(int k, int g) { return k - g < kTorRecFree ? k - g : kTorRecFree; }
+// Pattern p over the first g2 modes of an item that starts at pattern `lo` of the first g: the
+// other g2 - g modes, above them in the word, change fastest.
+__host__ __device__ inline uint32_t tor_rec_pattern(unsigned long long lo, unsigned long long p, int g, int g2) {
+  const int more = g2 - g;
+  return (uint32_t)((lo + (p >> more)) | ((p & ((1ull << more) - 1)) << g));
+}
 // Workspace (doubles) of an instance of k modes whose items fix the first g.
 __host__ __device__ inline int tor_rec_ws(int k, int g, bool is_dd, bool cert) {
   const int t = tor_rec_layout(k, tor_rec_free(k, g), is_dd ? TorRec<dd>::kTail : TorRec<double>::kTail, cert,

@@ -122,4 +122,37 @@ def test_certified_ladder_escalates_to_dd(gpu):
         assert d[i]["rel_error_bound"] <= 1e-10
         if d[i]["tier"] == "certified-dd":
             assert d[i]["escalated"] is True and v[i] == dd[i]
+
+
+@pytest.mark.parametrize("n", [16, 17])
+def test_splits_with_more_free_modes_than_one_walk_takes(gpu, lib, orc, n):
+    # 2^10 and 2^11 leaves per item leave 15 and 16 modes free, and 14 are walked at a time: 2
+    # or 4 walks per item, at 17 modes and 2^11 with a pattern of its own in each item; the
+    # same for 2^11 leaves in double-double
+    mats = np.stack([phys_O(n), phys_O(n, 3.0)])
+    want = gpu.tor_batched(mats, precision="dd") if n > 16 else np.array([orc.tor(m, "quad") for m in mats])
+    dd0 = gpu.tor_batched(mats, precision="dd")
+    _, diag = gpu.tor_batched(mats, precision="auto", return_diagnostics=True)
+    kappa = np.array([d["cancellation"] for d in diag])
+    cm = np.ascontiguousarray(mats, dtype=np.complex128)
+    out, bnd = np.empty(2, np.complex128), np.empty(2)
+    for split in (10, 11):
+        assert lib.gbs_set_split(3, 0, 2 * n, split, 0) == 0 and lib.gbs_set_split(3, 1, 2 * n, split, 0) == 0
+        try:
+            v = gpu.tor_batched(mats)
+            cv, cb = _cert(gpu, mats)
+            _, dk = gpu.tor_batched(mats, precision="auto", return_diagnostics=True)
+            dd = gpu.tor_batched(mats, precision="dd")
+            gpu._lib.check(lib.gbs_tor_dd_certified_host(gpu._lib.dptr(cm.view(np.float64)), n, 2,
+                                                         gpu._lib.dptr(out.view(np.float64)), gpu._lib.dptr(bnd)),
+                           "gbs_tor_dd_certified_host")
+        finally:
+            lib.gbs_set_split(3, 0, 2 * n, -1, 0)
+            lib.gbs_set_split(3, 1, 2 * n, -1, 0)
+        assert np.array_equal(v, cv) and np.array_equal(dd, out), split
+        assert (np.abs(cv - want) <= cb).all() and (np.abs(out - want) <= bnd).all(), split
+        assert (np.abs(v - want) <= 1e-15 * kappa * np.abs(want)).all(), split
+        # the double-double sum's own error, kappa 2^-104 or so, is below its rounding
+        assert (np.abs(dd - dd0) <= (2.0 ** -52 + 1e-28 * kappa) * np.abs(dd0)).all(), split
+        assert np.array([d["cancellation"] for d in dk]) == pytest.approx(kappa, rel=1e-6), split
     assert any(x["tier"] == "certified-dd" for x in d)  # click patterns cancel beyond binary64

@@ -70,8 +70,15 @@ def test_accesses_stay_inside_the_workspace(torlib, k):
                 g = k - f
                 for lo in (0, (1 << g) - 1, (0x55555555 & ((1 << g) - 1))):
                     _item(torlib, O, g, lo, is_dd, cert)
-    if k <= 17:
-        _item(torlib, O, 0, 0, 0, 1)  # more free modes than are walked at a time
+
+
+@pytest.mark.parametrize("k,g", [(15, 0), (16, 1), (16, 0)])
+def test_more_free_modes_than_are_walked_at_a_time(torlib, orc, k, g):
+    O = _phys_O(k, k)
+    t, absn = orc.tor(O.astype(complex), "quad", with_absnorm=True)
+    for is_dd in (0, 1):
+        v = sum(_item(torlib, O, g, lo, is_dd, 1) for lo in range(1 << g))
+        assert abs(v - t.real) <= 64 * k * k * 2.0 ** -53 * absn, is_dd
 
 
 @pytest.mark.parametrize("k", [2, 5, 6, 9])

@@ -97,10 +97,9 @@ extern "C" int t_tor_rec_item(const double* O, int k, int g, unsigned lo, int is
     }
   if (R.lc & 1) ++x.bad;  // column pairs on 16 bytes
   double sum = 0.0;
-  const unsigned subs = 1u << (k - f - g);
-  for (unsigned sub = 0; sub < subs; ++sub) {
-    const unsigned pat = lo | (sub << g);
-    const int g2 = k - f;
+  const int g2 = k - f;
+  for (unsigned p = 0; p < (1u << (g2 - g)); ++p) {
+    const unsigned pat = tor_rec_pattern(lo, p, g, g2);
     x.w.assign(R.rho, 0.0);
     x.set.assign(R.rho, 0);
     for (int e = 0; e < tor_rec_entries(k); ++e) {
