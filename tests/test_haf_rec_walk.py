@@ -2,7 +2,8 @@
 kernel's own layout, lane and node functions drive a sequential walk
 (tests/rec_host.cu) whose every access must lie inside the workspace the planner asks
 for and read a written word, for every split into blocks, and whose sums must equal the
-oracle's hafnian / loop hafnian."""
+oracle's hafnian / loop hafnian.  The double-double walk's layout and steps too: there no
+lane may touch a word that another one writes before the next barrier."""
 
 from __future__ import annotations
 
@@ -32,16 +33,16 @@ def reclib():
                "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(csrc), str(src), "-o", str(out)]
         subprocess.run(cmd, check=True, capture_output=True)
     lib = ctypes.CDLL(str(out))
-    lib.t_haf_rec_sum.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_uint, ctypes.c_int,
-                                  ctypes.c_void_p]
+    lib.t_haf_rec_sum.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_uint,
+                                  ctypes.c_int, ctypes.c_void_p]
     return lib
 
 
-def _sum(lib, A, loop, lo, clog):
+def _sum(lib, A, loop, is_dd, lo, clog):
     A = np.ascontiguousarray(A, dtype=np.complex128)
     out = np.zeros(2)
-    bad = lib.t_haf_rec_sum(A.ctypes.data, A.shape[0] // 2, int(loop), lo, clog, out.ctypes.data)
-    assert bad == 0, (A.shape, loop, lo, clog, bad)
+    bad = lib.t_haf_rec_sum(A.ctypes.data, A.shape[0] // 2, int(loop), is_dd, lo, clog, out.ctypes.data)
+    assert bad == 0, (A.shape, loop, is_dd, lo, clog, bad)
     return complex(out[0], out[1])
 
 
@@ -51,20 +52,22 @@ def _sym(N, seed):
     return (X + X.T) / 4
 
 
+@pytest.mark.parametrize("is_dd", [0, 1])
 @pytest.mark.parametrize("n", range(1, 11))
-def test_sums_equal_the_oracle_for_every_split(reclib, orc, n):
+def test_sums_equal_the_oracle_for_every_split(reclib, orc, n, is_dd):
     A = _sym(2 * n, n)
     for loop in (False, True):
         t, absn = getattr(orc, "lhaf" if loop else "haf")(A, "quad", with_absnorm=True)
         for clog in range(n + 1):
-            v = sum(_sum(reclib, A, loop, lo, clog) for lo in range(0, 1 << n, 1 << clog))
+            v = sum(_sum(reclib, A, loop, is_dd, lo, clog) for lo in range(0, 1 << n, 1 << clog))
             # the recursion's terms are smaller than the power trace's (absn), so their
             # rounding stays within a few n u of absn
             assert abs(v - t) <= 32 * n * 2.0 ** -53 * absn, (loop, clog)
 
 
+@pytest.mark.parametrize("is_dd", [0, 1])
 @pytest.mark.parametrize("n", [11, 12, 13, 14, 15, 16])
-def test_accesses_stay_inside_the_workspace(reclib, n):
+def test_accesses_stay_inside_the_workspace(reclib, n, is_dd):
     A = _sym(2 * n, n)
     g = np.random.default_rng(n)
     for loop in (False, True):
@@ -73,4 +76,4 @@ def test_accesses_stay_inside_the_workspace(reclib, n):
                 continue
             full = (1 << n) - (1 << clog)
             for lo in {0, full, int(g.integers(0, 1 << n)) & full, int(g.integers(0, 1 << n)) & full}:
-                _sum(reclib, A, loop, lo, clog)
+                _sum(reclib, A, loop, is_dd, lo, clog)
