@@ -52,13 +52,24 @@ def test_every_split_vs_oracle(gpu, lib, orc, N):
 
 @pytest.mark.parametrize("N", [30, 32])
 def test_largest_sizes_factorise(gpu, N):
-    """A direct sum: the hafnians of the blocks multiply (complex and real)."""
-    for real in (False, True):
+    """A direct sum: the hafnians of the blocks multiply (complex and real).  Proven bounds of
+    the factors and of the product have to meet; the binary64 value of these matrices errs by
+    4.5e-11 at most (measured; u times the sum of moduli of the power-trace terms is 8e-10 ..
+    3e-6), allowed four times that; the double-double one is good to its rounding."""
+    for real in (True, False):
         A, B = _mat(14, real, 1), _mat(N - 14, real, 2)
         blk = np.zeros((N, N), complex)
         blk[:14, :14], blk[14:, 14:] = A, B
         p = np.random.default_rng(3).permutation(N)
-        for f in ("haf", "lhaf"):
-            v, d = getattr(gpu, f)(blk[np.ix_(p, p)], precision="certified", return_diagnostics=True)
-            want = getattr(gpu, f)(A) * getattr(gpu, f)(B)
-            assert abs(v - want) <= d["abs_error_bound"] + 1e-9 * abs(want), (f, real, v, want)
+        blk = blk[np.ix_(p, p)]
+        for name in ("haf", "lhaf"):
+            f = getattr(gpu, name)
+            (v, d), (a, da), (b, db) = (f(X, precision="certified", return_diagnostics=True) for X in (blk, A, B))
+            ea, eb = da["abs_error_bound"], db["abs_error_bound"]
+            slack = abs(a) * eb + abs(b) * ea + ea * eb + 4 * U * abs(a * b)  # + the rounding of a * b
+            assert abs(v - a * b) <= d["abs_error_bound"] + slack, (name, real, v, a * b)
+            want = f(A, precision="dd") * f(B, precision="dd")  # good to a few u
+            kappa = f(blk, precision="auto", return_diagnostics=True)[1]["cancellation"]
+            assert abs(v - want) <= min(2e-10, U * kappa) * abs(want), (name, real, v, want, kappa)
+            vd = f(blk, precision="dd")
+            assert abs(vd - want) <= (8 * U + 1e-20 * kappa) * abs(want), (name, real, vd, want, kappa)
