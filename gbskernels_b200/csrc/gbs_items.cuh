@@ -281,7 +281,6 @@ __global__ void __launch_bounds__(256) gbs_items_kernel(ItemLaunch P) {
     if (lane == 0) it = atomicAdd(P.head, 1);
     it = __shfl_sync(0xffffffffu, it, 0);
     if (it >= n_items) break;
-    if (P.order) it = P.order[it];
     const WorkItem w = P.items[it];
     const InstDesc d = P.insts[w.inst];
     ItemResult r = eval_item<BR>(P, d, w, ws, lane);

@@ -60,8 +60,7 @@ constexpr unsigned kBrMixed = kBrServe | br1(kFnHaf, kTierDD) | br1(kFnLhaf, kTi
 struct ItemLaunch {
   const double* mats;      // packed matrices (complex interleaved; real-tor as complex too)
   const InstDesc* insts;
-  const WorkItem* items;
-  const int* order;        // optional queue order (item indices, heaviest first); null = identity
+  const WorkItem* items;   // in the order they are pulled
   int n_items;
   const int* n_items_dev = nullptr;  // optional: the item count, read on the device (a queue planned there)
   int* head;               // queue head (atomic), zeroed before launch

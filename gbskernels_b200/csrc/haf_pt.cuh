@@ -68,7 +68,7 @@ struct HafLayout {
   int slot;  // complex entries per ring slot (smax / 2 + 1)
   int c_off, p_off, y_off, d_off, gi_off, acc_off, ring_off, total;  // in doubles
 };
-__host__ __device__ inline HafLayout haf_layout(int smax, bool /* one layout for every tier */ = false) {
+__host__ __device__ inline HafLayout haf_layout(int smax) {
   HafLayout L;
   if (smax < 2) smax = 2;
   L.smax = smax;

@@ -703,7 +703,6 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     L.mats = (const double*)s->mats.p;
     L.insts = (const InstDesc*)dm;
     L.items = (const WorkItem*)(dm + ni * sizeof(InstDesc));
-    L.order = nullptr;
     L.n_items = nit;
     L.head = (int*)((char*)s->head.p + 64 * g);
     L.done = (int*)((char*)s->head.p + heads) + noff;

@@ -182,7 +182,6 @@ int gbs_haf_noalloc(const double* d_mats, int N, int batch, double* d_out, void*
   L.mats = d_mats;
   L.insts = d_insts;
   L.items = d_items;
-  L.order = nullptr;
   L.n_items = (int)nit;
   L.head = d_head;
   L.done = d_done;

@@ -367,7 +367,6 @@ int sampler_chain(const double* h_Ak, long long ak_total, const int* h_off, int 
   L.mats = B.sub.p;
   L.insts = B.insts.p;
   L.items = B.items.p;
-  L.order = nullptr;
   L.head = B.head.p;
   L.done = B.done.p;
   L.part = B.part.p;

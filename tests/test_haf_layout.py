@@ -1,12 +1,11 @@
-"""The hafnian workspace layout holds every access of the binary64 power loop.
+"""The layout of the indicator's power traces holds every access of the power loop.
 
 On the 8-tile path the power loop stores and reads whole live column tiles (the
 columns s .. 4 ntn - 1 hold zeros) and d is zero-padded to whole tiles, so the
 loop stays inside the warp's shared workspace only if the strides and regions of
 `haf_layout` are large enough for every subset size of a launch.  The layout
 functions are __host__ __device__; tests/layout_host.cu compiles them for the host
-and checks every (launch maximum, subset size) pair up to the cap, plain and
-certified.  Needs nvcc (present wherever the library is built) but no GPU."""
+and checks every (launch maximum, subset size) pair up to the cap.  Needs nvcc (present wherever the library is built) but no GPU."""
 
 from __future__ import annotations
 
