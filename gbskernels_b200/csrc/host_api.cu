@@ -136,7 +136,7 @@ struct ScatterArgs {
   int write_aux;
 };
 cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t st);
-cudaError_t launch_expand_real(const double* in, double* out, long long n, cudaStream_t st);
+cudaError_t launch_expand_real(const double* in, double* out, long long n, int sms, cudaStream_t st);
 
 struct Plan {
   std::vector<InstDesc> insts;
@@ -669,7 +669,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
       if (real_upload) {
         e = cudaMemcpyAsync(s->real.p, s->pin_in.p, mat_doubles / 2 * sizeof(double), cudaMemcpyHostToDevice, s->stream);
         if (e == cudaSuccess)
-          e = launch_expand_real((const double*)s->real.p, (double*)s->mats.p, mat_doubles / 2, s->stream);
+          e = launch_expand_real((const double*)s->real.p, (double*)s->mats.p, mat_doubles / 2, s->sms, s->stream);
       } else {
         e = cudaMemcpyAsync(s->mats.p, s->pin_in.p, mat_doubles * sizeof(double), cudaMemcpyHostToDevice, s->stream);
       }
@@ -1566,8 +1566,8 @@ int gbs_queue_run(gbs_session* s, void* stream) {
 }
 
 // Autotuner hooks: split = log2 of the work per item (haf / lhaf: subsets per item;
-// perm: Gray steps per lane; tor: prefix leaves per item, or subsets per lane in the
-// double-double tier); warps = block size of per-size launches; -1 / 0 = default.
+// perm: Gray steps per lane; tor: blocks of 32 subsets per item, 16 in the double-double
+// tiers); warps = block size of per-size launches; -1 / 0 = default.
 int gbs_set_split(int func, int tier, int dim, int split, int warps) {
   if (func < 0 || func > 3 || tier < 0 || tier > 4 || dim < 0 || dim >= kTuneDims || split < -1 || split > 40 ||
       warps < 0 || warps > 8)

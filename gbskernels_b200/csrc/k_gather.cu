@@ -97,8 +97,8 @@ __global__ void expand_real_kernel(const double* __restrict__ in, double2* __res
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = make_double2(in[i], 0.0);
 }
 
-cudaError_t launch_expand_real(const double* in, double* out, long long n, cudaStream_t st) {
-  const int grid = (int)std::min<long long>((n + 255) / 256, 148 * 8);
+cudaError_t launch_expand_real(const double* in, double* out, long long n, int sms, cudaStream_t st) {
+  const int grid = (int)std::min<long long>((n + 255) / 256, 8ll * sms);  // 8 blocks fill an SM
   expand_real_kernel<<<grid, 256, 0, st>>>(in, reinterpret_cast<double2*>(out), n);
   return cudaGetLastError();
 }
