@@ -28,7 +28,7 @@ import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
 EXT_DIR = ROOT / "gbskernels_b200" / "ext"
-REF = Path(os.environ.get("GBS_REFERENCE_DIR", "/root/reference"))
+REF = Path(os.environ.get("GBS_REFERENCE_DIR", ROOT.parent / "reference"))
 
 pytestmark = pytest.mark.skipif(not (REF / "gbskernels" / "__init__.py").exists(),
                                 reason="no reference checkout")
