@@ -9,7 +9,7 @@ per-size mode (one launch per bucket, the session's CUDA-event kernel time of th
 last of `reps` runs) and keeps the fastest:
 
   * split -- log2 of the work per item: haf / lhaf subsets per item, perm Gray steps
-    per lane, tor prefix leaves per item (32 tail subsets each); more work per item
+    per lane, tor blocks of 32 (double-double 16) subsets per item; more work per item
     means fewer items (less queue and reduction overhead) but coarser load balance;
   * warps -- warps per block of the per-size launches (1, 2 or 4), where the
     workspace allows more than one.

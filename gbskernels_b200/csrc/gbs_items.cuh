@@ -98,8 +98,8 @@ __device__ ItemResult perm_item(const double* __restrict__ mats, const InstDesc&
 }
 
 // REAL: the instance is real (binary64 tiers; the host sets InstDesc::real_in) and
-// runs the real power loop.  A separate instantiation, so the complex code is
-// compiled as if the real path did not exist.
+// runs the recursion over pairs in real arithmetic.  A separate instantiation, so the
+// complex code is compiled as if the real path did not exist.
 template <int TIER, bool REAL = false>
 __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, const InstDesc& d, const WorkItem& w,
                                bool loop, double* ws, int haf_smax, int lane) {

@@ -1,5 +1,5 @@
 // perm_tor.cuh -- permanent (Glynn / Gray code) work-item evaluators, binary64 and
-// double-double.  (The torontonian walks live in tor_warp.cuh / tor_warp_dd.cuh.)
+// double-double.  (The torontonian's walk lives in tor_rec.cuh, a complex one's in tor_lu.cuh.)
 //
 // Permanent (reference: cpu_ref/permanent.py:108-139, core/permanent.cu:30-76):
 //   perm(A) = 2^-(n-1) sum_{delta, delta_0 = +1} (prod delta) prod_r sum_c delta_c A[r][c],

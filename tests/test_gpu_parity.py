@@ -132,7 +132,7 @@ def test_lhaf_vs_binary128_oracle(gpu, orc, N):
 
 @pytest.mark.parametrize("N", [2, 4, 5, 6, 8, 9, 10, 12, 14, 16, 18, 20])
 def test_real_inputs_vs_binary128_oracle(gpu, orc, N):
-    """A real matrix (every imaginary part zero) runs the real power loop (real
+    """A real matrix (every imaginary part zero) runs the real recursion (real
     m16n8k8 products, K = s): hafnian (even N) and loop hafnian (odd N augmented)
     against binary128, in fp64 and in the indicator and certified tiers, whose
     values are the fp64 value bit for bit and whose radius encloses the truth."""

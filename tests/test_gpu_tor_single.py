@@ -1,7 +1,7 @@
 """Single-large torontonian (one instance over the whole GPU, up to 32 modes)
 against the binary128 oracle at small sizes and, past the batched cap, through the
 direct-sum identity tor(O1 (+) O2) = tor(O1) tor(O2) with the halves evaluated by
-the independent double-double kernel.  Reference test model:
+the double-double tier.  Reference test model:
 tests/test_torontonian.py (single-large rows) and tests/test_certified.py."""
 
 from __future__ import annotations

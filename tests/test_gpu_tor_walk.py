@@ -1,10 +1,9 @@
-"""Torontonian binary64 tiers (warp-cooperative prefix walk + 32-subset register
-tail) at every size class the decomposition distinguishes: k < 5 (tail only), k = 5
-(empty prefix), one-item instances, and multi-item instances for both the binary64
-decomposition (2^9 leaves per item) and the certified one (2^10), against the
-binary128 oracle, the independent double-double kernel (per-lane subtree walk) and
-the certified enclosures.  Reference test model: tests/test_torontonian.py and
-tests/test_certified.py (tor rows)."""
+"""Torontonian tiers (the recursion over modes on Schur complements) at every size class
+the walk distinguishes: k <= 4 (registers only), up to 9 (breadth-first levels), the
+depth-first part, one item, several items and several walks per item, against the
+binary128 oracle, the double-double tier (the same walk on double words, with its own
+split and tail) and the certified enclosures.  Reference test model:
+tests/test_torontonian.py and tests/test_certified.py (tor rows)."""
 
 from __future__ import annotations
 
@@ -48,7 +47,7 @@ def test_tor_sizes_vs_binary128(gpu, orc, n):
 @pytest.mark.parametrize("n", [14, 15, 16, 17])
 def test_tor_multi_item_vs_dd_kernel(gpu, n):
     # 14: one work item; 15/16/17: 2/4/8 items (every binary64 tier splits the same
-    # way).  The double-double kernel is a separate code path.
+    # way).  The double-double tier has another split and tail.
     mats = np.stack([phys_O(n) for _ in range(2)])
     _, diag = gpu.tor_batched(mats, precision="auto", return_diagnostics=True)
     dd = gpu.tor_batched(mats, precision="dd")
@@ -122,6 +121,7 @@ def test_certified_ladder_escalates_to_dd(gpu):
         assert d[i]["rel_error_bound"] <= 1e-10
         if d[i]["tier"] == "certified-dd":
             assert d[i]["escalated"] is True and v[i] == dd[i]
+    assert any(x["tier"] == "certified-dd" for x in d)  # click patterns cancel beyond binary64
 
 
 @pytest.mark.parametrize("n", [16, 17])
@@ -155,4 +155,3 @@ def test_splits_with_more_free_modes_than_one_walk_takes(gpu, lib, orc, n):
         # the double-double sum's own error, kappa 2^-104 or so, is below its rounding
         assert (np.abs(dd - dd0) <= (2.0 ** -52 + 1e-28 * kappa) * np.abs(dd0)).all(), split
         assert np.array([d["cancellation"] for d in dk]) == pytest.approx(kappa, rel=1e-6), split
-    assert any(x["tier"] == "certified-dd" for x in d)  # click patterns cancel beyond binary64

@@ -4,14 +4,12 @@ rest on, checked on the CPU.
 tor(O) = sum_{S subset [k]} (-1)^(k-|S|) / sqrt(det(I - O)_S)
 (cpu_ref/tor_recursive.py:46-100; xxpp indexing: mode i owns rows i and i + k).
 
-The warp walk (gbskernels_b200/csrc/tor_warp.cuh) splits the modes into a prefix
-of q = k - r modes, walked by the warp, and a tail of r modes whose 2^r subsets
-are the lanes.  At a prefix set S it holds the Schur complement of the whole tail,
-Z = M_TT - M_TS M_S^-1 M_ST (M = I - O), and lane T' factors Z restricted to the
-modes in T', so that det M_{S u T'} = det M_S * det Z_{T'}.  A lane factors Z
-with the rows of excluded modes read from an identity and their pivot reciprocal
-set to 0: every term those rows contribute is an exact zero, so the included
-entries see exactly the operations of the compressed factorisation.  These tests
+The recursion (gbskernels_b200/csrc/tor_rec.cuh) decides the modes one after the other.  At
+a set S of included modes it holds the Schur complement of the undecided ones T,
+Z = M_TT - M_TS M_S^-1 M_ST (M = I - O), shared by every subset below, since
+det M_{S u T'} = det M_S * det Z_{T'}.  Leaving a mode out is a view, including it one
+right-looking Cholesky step on its two rows, so that every entry sees the operations
+of the left-looking factorisation of its own minor, in the same order.  These tests
 check the decomposition against the oracle and that last claim bit for bit.
 """
 
@@ -67,53 +65,65 @@ def test_prefix_times_tail_schur_complement_is_the_torontonian(orc, k, r):
     assert abs(got - ref) <= 1e-11 * max(abs(ref), 1.0)
 
 
-def _chol_logdet_terms(Z: np.ndarray, include: list[bool]):
-    """Left-looking Cholesky in a fixed scalar order; rows with include False are
-    read from an identity and get pivot reciprocal 0.  Returns the pivots of the
-    included rows and the factor."""
-    n = Z.shape[0]
-    Zp = Z.copy()
+def _left_looking(A: np.ndarray) -> np.ndarray:
+    """The factor of one minor by itself, entry by entry."""
+    n = A.shape[0]
+    L, inv = np.zeros((n, n)), []
     for i in range(n):
-        if not include[i]:
-            Zp[i, :] = 0.0
-            Zp[:, i] = 0.0
-            Zp[i, i] = 1.0
-    L = np.zeros((n, n))
-    piv = []
-    for j in range(n):
-        s = float(Zp[j, j])
-        for t in range(j):
-            s = s - L[j, t] * L[j, t]
-        p = math.sqrt(s)
-        rinv = 1.0 / p if include[j] else 0.0
-        L[j, j] = p
-        if include[j]:
-            piv.append(p)
-        for i in range(j + 1, n):
-            x = float(Zp[i, j])
+        for j in range(i + 1):
+            x = float(A[i, j])
             for t in range(j):
                 x = x - L[i, t] * L[j, t]
-            L[i, j] = x * rinv
-    return piv, L
+            if j < i:
+                L[i, j] = x * inv[j]
+            else:
+                inv.append(1.0 / math.sqrt(x))
+                L[i, i] = inv[i]
+    return L
 
 
-@pytest.mark.parametrize("r", [3, 5])
-def test_packed_identity_rows_reproduce_the_compressed_factor_bit_for_bit(r):
-    k = r + 3
-    O = _O(k, seed=40 + r)
-    M = np.eye(2 * k) - O
-    it = _rows(range(k - r, k), k)
-    Z = M[np.ix_(it, it)]  # the tail block at the empty prefix (any SPD block will do)
-    for mt in range(r + 1):
-        for T in itertools.combinations(range(r), mt):
-            inc_modes = set(T)
-            include = [(i % r) in inc_modes for i in range(2 * r)]
-            piv_p, L_p = _chol_logdet_terms(Z, include)
-            sel = [i for i in range(2 * r) if include[i]]
-            piv_c, L_c = _chol_logdet_terms(Z[np.ix_(sel, sel)], [True] * len(sel))
-            assert [x.hex() for x in piv_p] == [x.hex() for x in piv_c]
-            sub = L_p[np.ix_(sel, sel)]
-            assert np.array_equal(sub.view(np.uint64), L_c.view(np.uint64))
+def _right_looking(Z: np.ndarray, modes, cols, out) -> None:
+    """Every subset of the modes that head Z (two rows each): leaving the first one out is a
+    view, including it gives the two columns (l, l') and Z'_ij = (Z_ij - l_i l_j) - l'_i l'_j.
+    `cols` holds the columns so far, by component; out[subset] = the factor's columns."""
+    if not modes:
+        out.append(cols)
+        return
+    _right_looking(Z[2:, 2:], modes[1:], cols, out)
+    n = Z.shape[0]
+    i0 = 1.0 / math.sqrt(Z[0, 0])
+    l0 = [float(Z[i, 0]) * i0 for i in range(n)]
+    i1 = 1.0 / math.sqrt(float(Z[1, 1]) - l0[1] * l0[1])
+    l1 = [0.0, 0.0] + [(float(Z[i, 1]) - l0[i] * l0[1]) * i1 for i in range(2, n)]
+    Y = np.zeros((n - 2, n - 2))
+    for i in range(2, n):
+        for j in range(2, i + 1):
+            Y[i - 2, j - 2] = (float(Z[i, j]) - l0[i] * l0[j]) - l1[i] * l1[j]
+    at = [(m, r) for m in modes for r in (0, 1)]
+    col0 = {c: l0[i] for i, c in enumerate(at)} | {at[0]: i0}
+    col1 = {c: l1[i] for i, c in enumerate(at) if i > 1} | {at[1]: i1}
+    _right_looking(Y, modes[1:], cols + [(modes[0], col0, col1)], out)
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 6])
+def test_shared_right_looking_steps_give_every_minors_own_factor_bit_for_bit(k):
+    M = np.eye(2 * k) - _O(k, seed=40 + k)
+    order = [i for j in range(k) for i in (j, j + k)]
+    found = []
+    _right_looking(M[np.ix_(order, order)], list(range(k)), [], found)
+    assert len(found) == 1 << k
+    for cols in found:
+        modes = [m for m, _, _ in cols]
+        comps = [(m, r) for m in modes for r in (0, 1)]
+        L = np.zeros((2 * len(modes), 2 * len(modes)))
+        for c, (_, col0, col1) in enumerate(cols):
+            for i, comp in enumerate(comps):
+                if i >= 2 * c:
+                    L[i, 2 * c] = col0[comp]
+                if i >= 2 * c + 1:
+                    L[i, 2 * c + 1] = col1[comp]
+        idx = [m + r * k for m, r in comps]
+        assert np.array_equal(L, _left_looking(M[np.ix_(idx, idx)]))
 
 
 # ---------------------------------------------------------------- permanent
@@ -159,14 +169,15 @@ def test_aligned_gray_ranges_sum_to_the_permanent(orc, n, rlog):
 
 
 # ---------------------------------------------------------------- repeated-row sieve
-# The sieve kernel (gbskernels_b200/csrc/k_sieve.cu) walks the digit vectors v of a
-# repetition pattern in reflected mixed-radix Gray order (digit 0 fastest, the
-# largest n_i on top with only floor(n_top / 2) + 1 values: the v <-> n - v
-# symmetry, weight 2 below the middle).  A work item restarts at Gray index t0 from
-# a directly decoded state: per digit q = t0 / place, b = q mod radix, reflected
-# (g = radix - 1 - b) when the parity of q / radix is odd, the top digit never
-# reflected.  A step moves the lowest digit that is not at the end of its run by
-# +-1 (the sign from its reflection parity) and resets the digits below it.
+# The sieve kernel (gbskernels_b200/csrc/k_sieve.cu) sums over the digit vectors v of a
+# repetition pattern (digit 0 fastest, the largest n_i on top with only
+# floor(n_top / 2) + 1 values: the v <-> n - v symmetry, weight 2 below the middle).  Its
+# lanes walk the few smallest digits in reflected mixed-radix Gray order from 0 and hold
+# one combination of the others each.  A term's digits follow from its place t in the walk
+# (the kernel tables the weights by that): per digit q = t / place, b = q mod radix,
+# reflected (g = radix - 1 - b) when q / radix is odd.  A step moves the lowest digit that
+# is not at the end of its run by +-1 (the sign from its reflection parity) and resets the
+# digits below it.  Checked here on walks of all digits, the top one never reflected.
 
 
 def _sieve_digits(reps):

@@ -73,7 +73,7 @@ def test_noalloc_matches_host_entry_point_twice(lib):
 
 
 def test_noalloc_real_input_agrees_to_rounding(lib):
-    # a real input runs the real power loop through gbs_haf_host and the complex one
+    # a real input runs the real recursion through gbs_haf_host and the complex one
     # here: equal to rounding, not bit for bit
     rng = np.random.default_rng(31)
     for N in (12, 20):
