@@ -203,12 +203,6 @@ __host__ __device__ inline TorRecState tor_rec_walked(const TorRecLayout& R, con
   return TorRecState{tor_rec_dfs(R, R.mW + s), R.f - (R.mW + s)};
 }
 
-// ------------------------------------------------------------------ scalars
-__device__ __forceinline__ double ts_ld(const double* ws, int i, double) { return ws[i]; }
-__device__ __forceinline__ dd ts_ld(const double* ws, int i, dd) { return ld_dd(ws + 2 * i); }
-__device__ __forceinline__ void ts_st(double* ws, int i, double v) { ws[i] = v; }
-__device__ __forceinline__ void ts_st(double* ws, int i, dd v) { st_dd(ws + 2 * i, v); }
-__device__ __forceinline__ double ts_fms(double a, double b, double c) { return fma(-b, c, a); }
 // The entry of O read for row i, column j <= i of M.  O is meant to be symmetric; of one that
 // is not, the torontonian reads the lower triangle in the order (mode, x before p), as the
 // reference does, but for the block of the last `tail` modes (5, double-double 4) against the
@@ -220,6 +214,12 @@ __host__ __device__ inline void tor_rec_source(int k, int tail, int i, int j, in
   row = upper ? a : b;
   col = upper ? b : a;
 }
+// ------------------------------------------------------------------ scalars
+__device__ __forceinline__ double ts_ld(const double* ws, int i, double) { return ws[i]; }
+__device__ __forceinline__ dd ts_ld(const double* ws, int i, dd) { return ld_dd(ws + 2 * i); }
+__device__ __forceinline__ void ts_st(double* ws, int i, double v) { ws[i] = v; }
+__device__ __forceinline__ void ts_st(double* ws, int i, dd v) { st_dd(ws + 2 * i, v); }
+__device__ __forceinline__ double ts_fms(double a, double b, double c) { return fma(-b, c, a); }
 __device__ __forceinline__ dd ts_fms(dd a, dd b, dd c) { return dd_fms(a, b, c); }
 __device__ __forceinline__ double ts_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ dd ts_mul(dd a, dd b) { return dd_mul(a, b); }
