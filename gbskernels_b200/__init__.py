@@ -64,7 +64,12 @@ def _check_backend(backend: str) -> None:
 def _as_stack(matrices: Iterable[Any]) -> np.ndarray:
     """The batch as a C-contiguous (B, d, d) array: float64 for real input (the library
     takes it as it is), complex128 otherwise."""
-    arr = np.asarray(matrices)
+    first = matrices
+    while type(first) in (list, tuple) and first:
+        first = first[0]
+    # a batch that starts with a complex number needs no look at the rest to know its type
+    starts_complex = isinstance(first, complex) or getattr(getattr(first, "dtype", None), "kind", "") == "c"
+    arr = np.asarray(matrices, dtype=np.complex128 if starts_complex else None)
     real = arr.dtype.kind in "fiub" and arr.dtype.itemsize <= 8
     if not real and arr.dtype.kind not in "cf":  # objects, texts: numpy's own conversion of the input
         arr = np.asarray(matrices, dtype=np.complex128)

@@ -34,6 +34,15 @@ def test_a_list_is_converted_once(G, dtype):
     assert _conversions(G._as_stack, mats) == once
 
 
+@pytest.mark.parametrize("wrap", [list, tuple, lambda s: s.tolist(), lambda s: [list(m) for m in s]])
+def test_a_complex_list_is_read_once_as_complex(G, monkeypatch, wrap):
+    # the type of nested lists costs numpy as much to find as the numbers to read
+    batch, seen, asarray = wrap(np.arange(18.0).reshape(2, 3, 3) + 1j), [], np.asarray
+    monkeypatch.setattr(G.np, "asarray", lambda a, dtype=None: (seen.append(dtype), asarray(a, dtype=dtype))[1])
+    G._as_stack(batch)
+    assert seen == [np.complex128]
+
+
 @pytest.mark.parametrize("dtype", [np.complex128, np.complex64, np.clongdouble, np.longdouble, np.float64, np.float32,
                                    np.float16, np.int64, np.uint8, bool, object, "U32"])
 def test_a_list_gives_the_numbers_of_its_stack(G, dtype):
