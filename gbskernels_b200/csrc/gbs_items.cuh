@@ -118,36 +118,38 @@ __device__ __noinline__ ItemResult haf_item(const double* __restrict__ mats, con
       if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
     }
   } else {
-    // binary64 tiers: the recursion over pairs (haf_rec.cuh)
-    using Z = std::conditional_t<REAL, double, cplx>;
-    bool tiny = false;
-    const Z v = haf_rec_sum<Z, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
-    // a real value that is not finite is NaN in both parts, as in complex arithmetic
-    if constexpr (REAL) r.val = ddc_from_c(isfinite(v) ? mkc(v, 0.0) : mkc(NAN, NAN));
-    else r.val = ddc_from_c(v);
-    if (TIER == kTierCert) {
-      const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
-      r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj, false);
-      // a halving that could round absolutely refuses the certificate
-      if (__any_sync(0xffffffffu, tiny)) r.aux = INFINITY;
-      if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
-    } else if (TIER == kTierKappa) {
+    if constexpr (TIER != kTierTerms) {
+      // binary64 tiers: the recursion over pairs (haf_rec.cuh)
+      using Z = std::conditional_t<REAL, double, cplx>;
+      bool tiny = false;
+      const Z v = haf_rec_sum<Z, false>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+      // a real value that is not finite is NaN in both parts, as in complex arithmetic
+      if constexpr (REAL) r.val = ddc_from_c(isfinite(v) ? mkc(v, 0.0) : mkc(NAN, NAN));
+      else r.val = ddc_from_c(v);
+      if (TIER == kTierCert) {
+        const double maj = haf_rec_sum<double, true>(A, N, loop, (unsigned)w.lo, (unsigned)w.count, ws, lane, tiny);
+        r.aux = haf_rec_radius(n, loop, (unsigned)w.count, maj, false);
+        // a halving that could round absolutely refuses the certificate
+        if (__any_sync(0xffffffffu, tiny)) r.aux = INFINITY;
+        if (!isfinite(r.aux) || !isfinite(r.val.re.hi) || !isfinite(r.val.im.hi)) r.st = kStUncertified;
+      }
+    }
+    if constexpr (TIER == kTierKappa || TIER == kTierTerms) {
       // the cancellation indicator is the sum of the moduli of the subsets' power-trace
-      // terms, so those are evaluated beside the value (haf_pt.cuh)
+      // terms, evaluated beside the value, or without it for an instance of the terms
+      // alone (haf_pt.cuh)
       const HafLayout L = haf_layout(haf_smax);
       double* ring = ws + L.ring_off;
-      double absacc = 0.0;
       int cnt = 0;
       for (unsigned long long k = 0; k < w.count; ++k) {
         haf_subset_traces<REAL>(A, N, n, (uint32_t)(w.lo + k), loop, ws, L, lane, ring + cnt * L.slot * 2);
         if (++cnt == kHafRing || k + 1 == w.count) {
           __syncwarp();
-          absacc += haf_ring_flush(ring, L.slot, cnt, n, lane, ws + L.p_off);
+          r.aux += haf_ring_flush(ring, L.slot, cnt, n, lane, ws + L.p_off);
           cnt = 0;
           __syncwarp();
         }
       }
-      r.aux = absacc;
     }
   }
   return r;
@@ -250,6 +252,8 @@ __device__ __forceinline__ ItemResult eval_item(const ItemLaunch& P, const InstD
     GBSB_BR(kFnHaf, kTierDD, (haf_item<kTierDD>(P.mats, d, w, false, ws, P.haf_smax, lane)))
     GBSB_BR(kFnLhaf, kTierFp64, (GBSB_HAF(kTierFp64, true)))
     GBSB_BR(kFnLhaf, kTierKappa, (GBSB_HAF(kTierKappa, true)))
+    GBSB_BR(kFnHaf, kTierTerms, (GBSB_HAF(kTierTerms, false)))
+    GBSB_BR(kFnLhaf, kTierTerms, (GBSB_HAF(kTierTerms, true)))
     GBSB_BR(kFnLhaf, kTierDD, (haf_item<kTierDD>(P.mats, d, w, true, ws, P.haf_smax, lane)))
     GBSB_BR(kFnTor, kTierFp64, (tor_item<kTierFp64>(P.mats, d, w, ws, lane)))
     GBSB_BR(kFnTor, kTierKappa, (tor_item<kTierKappa>(P.mats, d, w, ws, lane)))
@@ -271,7 +275,7 @@ __device__ __forceinline__ ItemResult eval_item(const ItemLaunch& P, const InstD
 }
 
 template <unsigned BR>
-__global__ void __launch_bounds__(256) gbs_items_kernel(ItemLaunch P) {
+__global__ void __launch_bounds__(BR == kBrTerms ? 384 : 256) gbs_items_kernel(ItemLaunch P) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   double* ws = smem + (size_t)warp * P.ws_doubles;

@@ -17,6 +17,8 @@ namespace gbsb {
 enum : int { kFnPerm = 0, kFnHaf = 1, kFnLhaf = 2, kFnTor = 3 };
 // tier codes (kTierCertDD: double-double value + rigorous bound)
 enum : int { kTierFp64 = 0, kTierDD = 1, kTierKappa = 2, kTierCert = 3, kTierCertDD = 4 };
+// the planner's own: the sum of a hafnian's indicator terms without its value
+constexpr int kTierTerms = 5;
 
 __host__ __device__ constexpr int ft_code(int fn, int tier) { return fn * 8 + tier; }
 __host__ __device__ constexpr int ft_fn(int ft) { return ft >> 3; }
@@ -43,11 +45,21 @@ struct WorkItem {       // 24 bytes
 // log2 of the subsets per hafnian / loop-hafnian work item in the binary64 tiers
 // (the planner and the allocation-free entry share it, so values agree bit for bit)
 constexpr int kHafItemLog2 = 7;
+// Indicator terms of hafnians with more pairs than this run in a launch of their own, in items
+// of 2^kTermsItemLog2 subsets, each a chain of matrix powers (8 us of a warp at side 20);
+// up to here value and terms are one item.
+constexpr int kTermsItemLog2 = 5;
 
 // Branch sets compiled into an item kernel (bit ft_code).  A launch uses the
 // smallest compiled set covering the (function, tier) pairs of its batch.
 constexpr unsigned br1(int fn, int tier) { return 1u << ft_code(fn, tier); }
 constexpr unsigned kBrHafLhafFp64 = br1(kFnHaf, kTierFp64) | br1(kFnLhaf, kTierFp64);
+// the indicator terms of hafnians and loop hafnians (a launch of their own beside the values):
+// on 168 registers a thread, for the sizes whose workspaces let 12 warps onto an SM (2,000
+// complex 20 x 20: terms 11.4 ms against 13.6 with 10 warps), or on all it wants, 198, for the
+// others (64 complex 28 x 28, 8 warps: 16.8 ms against 17.5)
+constexpr unsigned kBrTerms = br1(kFnHaf, kTierTerms) | br1(kFnLhaf, kTierTerms);
+constexpr unsigned kBrTermsLarge = kBrTerms | 1u << 31;
 // haf / lhaf / tor in fp64, fp64 + indicator and certified: the serving mix
 constexpr unsigned kBrServe = kBrHafLhafFp64 | br1(kFnTor, kTierFp64) | br1(kFnHaf, kTierKappa) |
                               br1(kFnLhaf, kTierKappa) | br1(kFnTor, kTierKappa) | br1(kFnHaf, kTierCert) |

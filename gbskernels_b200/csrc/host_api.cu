@@ -43,6 +43,7 @@ GBSB_DECL_GROUP(perm_fp64)
 GBSB_DECL_GROUP(perm_kappa)
 GBSB_DECL_GROUP(perm_dd)
 GBSB_DECL_GROUP(haf)
+GBSB_DECL_GROUP(terms)
 GBSB_DECL_GROUP(haf_dd)
 GBSB_DECL_GROUP(tor)
 GBSB_DECL_GROUP(mixed)
@@ -56,6 +57,7 @@ static cudaError_t launch_any(unsigned br, const ItemLaunch& P, int grid, int wa
   if (items_launch_perm_kappa(br, P, grid, warps, s, &e)) return e;
   if (items_launch_perm_dd(br, P, grid, warps, s, &e)) return e;
   if (items_launch_haf(br, P, grid, warps, s, &e)) return e;
+  if (items_launch_terms(br, P, grid, warps, s, &e)) return e;
   if (items_launch_haf_dd(br, P, grid, warps, s, &e)) return e;
   if (items_launch_tor(br, P, grid, warps, s, &e)) return e;
   if (items_launch_mixed(br, P, grid, warps, s, &e)) return e;
@@ -69,6 +71,7 @@ static int occ_any(unsigned br, const ItemLaunch& P, int warps) {
   if ((r = items_occ_perm_kappa(br, P, warps)) >= 0) return r;
   if ((r = items_occ_perm_dd(br, P, warps)) >= 0) return r;
   if ((r = items_occ_haf(br, P, warps)) >= 0) return r;
+  if ((r = items_occ_terms(br, P, warps)) >= 0) return r;
   if ((r = items_occ_haf_dd(br, P, warps)) >= 0) return r;
   if ((r = items_occ_tor(br, P, warps)) >= 0) return r;
   if ((r = items_occ_mixed(br, P, warps)) >= 0) return r;
@@ -78,6 +81,7 @@ static int occ_any(unsigned br, const ItemLaunch& P, int warps) {
 }
 // Smallest compiled branch set covering `need`.
 static unsigned cover(unsigned need) {
+  if (need & kBrTerms) return kBrTerms;  // never beside others
   if (__builtin_popcount(need) == 1) return need;
   const unsigned sets[] = {kBrHafLhafFp64, kBrServe, kBrMixed};
   for (unsigned s : sets)
@@ -193,9 +197,11 @@ static Split split_of(int fn, int tier, int dim_eval, bool real_in, int split) {
   } else if (fn == kFnHaf || fn == kFnLhaf) {
     const int n = dim_eval / 2;
     S.total = 1ull << n;
-    // masks per item: 2^kHafItemLog2 (binary64 tiers) / 2^6 (double-double); smaller instances are one item
+    // masks per item: 2^kHafItemLog2 (binary64 tiers) / 2^6 (double-double); smaller instances are
+    // one item.  The indicator's terms, whose sum is no one's value, have a split of their own.
     int per = is_dd ? std::min(n, 6) : std::min(n, kHafItemLog2);  // dd tiers: one split
     if (tl >= 0) per = std::min(n, tl);
+    if (tier == kTierTerms) per = std::min(n, kTermsItemLog2);
     S.count = 1ull << per;
   } else if (!real_in) {  // tor, complex O: ranges of subset masks, one LU per subset
     const int n = dim_eval / 2;
@@ -228,15 +234,15 @@ static double item_cost(int fn, int dim, int tier, const Split& S) {
     case kFnTor:
       c = S.param < 0 ? count * dim * dim * dim : count * std::ldexp(120.0, dim / 2 - S.param);
       break;
-    default:  // recursion over pairs; the indicator tier runs power traces too
-      c = count * 12.0 * n * n * (fn == kFnLhaf ? 1.9 : 1.0);
-      if (tier == kTierKappa) c += count * (n + 1) * n * n * n;
+    default:  // recursion over pairs; the indicator's terms by power traces
+      c = tier == kTierTerms ? 0.0 : count * 12.0 * n * n * (fn == kFnLhaf ? 1.9 : 1.0);
+      if (tier == kTierKappa || tier == kTierTerms) c += count * (n + 1) * n * n * n;
   }
   return is_dd ? 20.0 * c : c;
 }
 
 // split_of and item_cost of the last request asked for: the requests of a batch mostly repeat
-// (2,000 permanents 2 x 2: 172 us a call with every split computed twice, 162 us before).
+// (2,000 permanents 2 x 2: 154 us a call, 172 with every split computed twice).
 struct Cut {
   int fn = -1, tier = 0, dim = 0, split = 0;
   bool real_in = false;
@@ -270,7 +276,8 @@ static int plan_instance(Plan& P, int fn, int tier, int dim_eval, bool real_in, 
     w.count = std::min(S.count, S.total - lo);
     P.items.push_back(w);
   }
-  if (fn == kFnHaf || fn == kFnLhaf) P.haf_smax = std::max(P.haf_smax, dim_eval);
+  if ((fn == kFnHaf || fn == kFnLhaf) && (tier == kTierKappa || tier == kTierTerms))
+    P.haf_smax = std::max(P.haf_smax, dim_eval);
   d.nitems = (int)P.items.size() - d.item0;
   P.insts.push_back(d);
   P.need |= 1u << d.ft;
@@ -302,8 +309,8 @@ static int ws_for_plan(const Plan& P) {
       w = tor_rec_ws(d.dim / 2, d.param, tier == kTierDD || tier == kTierCertDD, tier_certified(tier));
     else {
       const int width = tier == kTierDD || tier == kTierCertDD ? 4 : (d.real_in ? 1 : 2);
-      w = rec_ws(d.dim / 2, fn == kFnLhaf, width);
-      if (tier == kTierKappa)  // the power-trace terms use a workspace of the launch's largest side
+      if (tier != kTierTerms) w = rec_ws(d.dim / 2, fn == kFnLhaf, width);
+      if (tier == kTierKappa || tier == kTierTerms)  // the power traces: of their largest side in the launch
         w = std::max(w, haf_layout(P.haf_smax).total + (d.real_in ? haf_real_layout(P.haf_smax).total : 0));
     }
     ws = std::max(ws, w);
@@ -351,12 +358,14 @@ struct gbs_session {
     int ni = 0, nit = 0;
     size_t out_off = 0;     // instance offset into the session's result arrays
     std::vector<int> req;   // request index of each instance
+    bool terms = false;     // indicator terms: the aux of requests whose values are in another group
   };
   std::vector<Group> groups;
   int plan_B = 0;
   std::vector<char> plan_trivial;
   std::vector<gbsb::cplx> plan_tval;
   std::vector<int> plan_tier;  // tier of each request
+  std::vector<char> plan_terms;  // request with indicator terms in a group of their own
   size_t plan_ninst = 0;
   bool plan_ready = false;
   // CUDA graph of the prepared plan's launch sequence (queue resets + one launch per
@@ -487,11 +496,19 @@ struct RunOpts {
   int warps = 4;           // warps per block
 };
 
+// Hafnians and loop hafnians of the indicator tier are two instances of one matrix: the value,
+// as in fp64, and the sum of the moduli of the power-trace terms (all but the smallest, where
+// an instance more costs more than it gives).
+static bool has_terms(const Req& r, int dim_eval) {
+  return r.tier == kTierKappa && (r.fn == kFnHaf || r.fn == kFnLhaf) && dim_eval / 2 > kTermsItemLog2;
+}
+
 // Build the device-resident plan of `reqs`: validate, pack and upload every matrix
 // once, cut the work items, upload the queue(s).  One group = one launch: a single
 // group holds every haf / lhaf / tor request (persistent mixed queue); the
-// permanent gets one group per tier; per-size mode gives one group per
-// (func, tier, size) bucket.
+// permanent gets one group per tier, the indicator terms of hafnians and loop hafnians one (in
+// the queue beside the recursion they had its registers and its workspace, 8 warps an SM
+// instead of 10 at side 20); per-size mode gives one group per (func, tier, size) bucket.
 static void drop_graph(gbs_session* s) {
   if (s->graph) cudaGraphExecDestroy(s->graph);
   s->graph = nullptr;
@@ -507,6 +524,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
   s->plan_trivial.assign(B, 0);
   s->plan_tval.assign(B, mkc(0, 0));
   s->plan_tier.assign(B, 0);
+  s->plan_terms.assign(B, 0);
   for (int i = 0; i < B; ++i) s->plan_tier[i] = reqs[i].tier;
   s->plan_ninst = 0;
   if (B == 0) { s->plan_ready = true; return 0; }
@@ -525,29 +543,44 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     if (!tr) mat_doubles += 2ll * dim_eval[i] * dim_eval[i];
   }
   std::vector<std::vector<int>> groups;
+  std::vector<char> gterms;
   if (opt.per_size) {
     std::vector<long long> keys;
     for (int i = 0; i < B; ++i) {
       if (s->plan_trivial[i]) continue;
-      long long key = ((long long)reqs[i].fn * 8 + reqs[i].tier) * 4096 + dim_eval[i];
-      size_t g = std::find(keys.begin(), keys.end(), key) - keys.begin();
-      if (g == keys.size()) { keys.push_back(key); groups.emplace_back(); }
-      groups[g].push_back(i);
+      s->plan_terms[i] = has_terms(reqs[i], dim_eval[i]);
+      for (int tier : {s->plan_terms[i] ? (int)kTierFp64 : reqs[i].tier, kTierTerms}) {
+        const long long key = ((long long)reqs[i].fn * 8 + tier) * 4096 + dim_eval[i];
+        size_t g = std::find(keys.begin(), keys.end(), key) - keys.begin();
+        if (g == keys.size()) {
+          keys.push_back(key);
+          groups.emplace_back();
+          gterms.push_back(tier == kTierTerms);
+        }
+        groups[g].push_back(i);
+        if (!s->plan_terms[i]) break;
+      }
     }
   } else {
-    groups.resize(6);  // everything but the permanent, then the permanent per tier (0..4)
+    groups.resize(7);  // everything but the permanent, the permanent per tier (0..4), the terms
+    gterms.assign(7, 0);
+    gterms[6] = 1;
     for (int i = 0; i < B; ++i) {
       if (s->plan_trivial[i]) continue;
+      s->plan_terms[i] = has_terms(reqs[i], dim_eval[i]);
       groups[reqs[i].fn == kFnPerm ? 1 + reqs[i].tier : 0].push_back(i);
+      if (s->plan_terms[i]) groups[6].push_back(i);
     }
   }
   // ---- plans of every group (host) and the sizes of the concatenated device arrays
   std::vector<Plan> plans;
   std::vector<std::vector<int>> greq;
-  for (auto& grp : groups) {
-    if (grp.empty()) continue;
+  std::vector<char> pterms;
+  for (size_t g = 0; g < groups.size(); ++g) {
+    if (groups[g].empty()) continue;
     plans.emplace_back();
-    greq.push_back(grp);
+    greq.push_back(std::move(groups[g]));
+    pterms.push_back(gterms[g]);
   }
   std::vector<long long> off(B, 0);
   {
@@ -561,9 +594,10 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
   size_t meta_bytes = 0, tot_items = 0, tot_inst = 0;
   for (size_t g = 0; g < plans.size(); ++g) {
     Plan& P = plans[g];
+    auto tier_of = [&](int i) { return !s->plan_terms[i] ? reqs[i].tier : (pterms[g] ? kTierTerms : (int)kTierFp64); };
     Cut cut;
     auto cut_of = [&](int i) -> const Cut& {
-      return cut.of(reqs[i].fn, reqs[i].tier, dim_eval[i], real_in[i] != 0, reqs[i].split);
+      return cut.of(reqs[i].fn, tier_of(i), dim_eval[i], real_in[i] != 0, reqs[i].split);
     };
     // heaviest instances first: the queue is pulled in item order
     if (opt.sort_heavy && !opt.per_size) {
@@ -584,7 +618,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
       P.items.reserve(nit);
       P.insts.reserve(c.size());
     }
-    for (int i : greq[g]) plan_instance(P, reqs[i].fn, reqs[i].tier, dim_eval[i], real_in[i], off[i], cut_of(i).S);
+    for (int i : greq[g]) plan_instance(P, reqs[i].fn, tier_of(i), dim_eval[i], real_in[i], off[i], cut_of(i).S);
     P.ws_doubles = ws_for_plan(P);
     const int ni = (int)P.insts.size(), nit = (int)P.items.size();
     if (cover(P.need) == 0) return fail(cudaErrorNotSupported, "no compiled kernel covers this mix");
@@ -744,13 +778,16 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     // reserves shared memory of its own, so small blocks can lose a warp)
     const size_t smem_per_warp = (size_t)P.ws_doubles * sizeof(double);
     int warps = opt.warps;
-    if (smem_per_warp >= 8192) {
+    if (smem_per_warp >= 8192 || pterms[g]) {
       int best = 0;
-      for (int w = 1; w <= 4; w <<= 1) {
-        if ((size_t)w * smem_per_warp > kMaxBlockSmem) break;
-        const int resident = occ_any(G.br, L, w) * w;
-        if (resident > best) { best = resident; warps = w; }
-      }
+      // (the terms' kernel with more registers first: the other one needs more warps to win)
+      const unsigned sets[] = {pterms[g] ? kBrTermsLarge : G.br, kBrTerms};
+      for (int k = 0; k < (pterms[g] ? 2 : 1); ++k)
+        for (int w = 1; w <= 4; w <<= 1) {
+          if ((size_t)w * smem_per_warp > kMaxBlockSmem) break;
+          const int resident = occ_any(sets[k], L, w) * w;
+          if (resident > best) { best = resident; warps = w; G.br = sets[k]; }
+        }
       if (best == 0) warps = 1;
     }
     if (opt.per_size && !P.insts.empty()) {  // a per-size bucket: the tuned block size, if any
@@ -767,6 +804,7 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
     G.nit = nit;
     G.out_off = noff;
     G.req = greq[g];
+    G.terms = pterms[g] != 0;
     s->groups.push_back(std::move(G));
     moff += ((ni * sizeof(InstDesc) + nit * sizeof(WorkItem)) + 255) & ~(size_t)255;
     ioff += nit;
@@ -861,9 +899,10 @@ static void plan_collect(gbs_session* s, double* out, double* aux, int* st) {
   for (const auto& G : s->groups)
     for (int k = 0; k < G.ni; ++k) {
       const int i = G.req[k];
+      if (aux && (G.terms || !s->plan_terms[i])) aux[i] = pa[G.out_off + k];
+      if (G.terms) continue;
       out[2 * i] = po[2 * (G.out_off + k)];
       out[2 * i + 1] = po[2 * (G.out_off + k) + 1];
-      if (aux) aux[i] = pa[G.out_off + k];
       if (st) st[i] = ps[G.out_off + k];
     }
   for (int i = 0; i < s->plan_B; ++i) {
@@ -906,8 +945,8 @@ static int plan_scatter(gbs_session* s, cudaStream_t stream, double* block, int 
   int* hm = (int*)s->pin_rmap.p;
   for (const auto& G : s->groups)
     for (int k = 0; k < G.ni; ++k) {
-      const int i = G.req[k];
-      hm[G.out_off + k] = remap ? (*remap)[i] : i;
+      const int i = G.req[k], to = remap ? (*remap)[i] : i;
+      hm[G.out_off + k] = !s->plan_terms[i] ? to : (G.terms ? ~(2 * to) : ~(2 * to + 1));
     }
   for (int t = 0; t < nt; ++t) hm[ni + t] = tidx[t];
   double* hv = (double*)(hm + ints);
@@ -1058,14 +1097,13 @@ static int one_shot(int fn, int tier, const double* m, int dim, int b, double* o
 
 // auto tier: fp64 + indicator, then the elements with kappa >= threshold rerun in
 // double-double on the device.  tier_out: 0 = fp64 kept, 1 = dd rerun.
-static int auto_batch(gbs_session* s, const std::vector<Req>& reqs, double kappa_max, double* out, double* kappa,
+static int auto_batch(gbs_session* s, std::vector<Req>&& reqs, double kappa_max, double* out, double* kappa,
                       int* tier_out, int* st) {
   const int B = (int)reqs.size();
-  std::vector<Req> kreq = reqs;
-  for (Req& r : kreq) r.tier = kTierKappa;
+  for (Req& r : reqs) r.tier = kTierKappa;
   std::vector<double> absn(B);
   RunOpts opt;
-  int rc = run_batch(s, kreq, out, absn.data(), st, opt);
+  int rc = run_batch(s, reqs, out, absn.data(), st, opt);
   if (rc) return rc;
   std::vector<Req> rerun;
   std::vector<int> idx;
@@ -1103,7 +1141,7 @@ static int auto_batch(gbs_session* s, const std::vector<Req>& reqs, double kappa
 static int session_reserve(gbs_session* s, size_t mat_bytes, size_t items, size_t insts) {
   items = std::max<size_t>(items, 1);
   insts = std::max<size_t>(insts, 1);
-  const size_t in = std::max<size_t>(mat_bytes, 16) + insts * sizeof(InstDesc) + items * sizeof(WorkItem) + 1024;
+  const size_t in = std::max<size_t>(mat_bytes, 16) + insts * sizeof(InstDesc) + items * sizeof(WorkItem) + 8 * 256;  // + a launch's padding each
   cudaError_t e = grow_pin(s->pin_in, in);
   if (e == cudaSuccess) e = grow_dev(s->mats, in, &s->reallocs);
   if (e == cudaSuccess) e = grow_dev(s->part, items * 4 * sizeof(double), &s->reallocs);
@@ -1306,10 +1344,10 @@ static int auto_host(int func, const double* m, int dim, int b, double kappa_max
   gbs_session* s;
   int rc = with_default(&s);
   if (rc) return rc;
-  const std::vector<Req> reqs = uniform_reqs(func, kTierFp64, m, dim, b, real_src);
+  std::vector<Req> reqs = uniform_reqs(func, kTierFp64, m, dim, b, real_src);
   std::vector<int> st(b);
   std::lock_guard<std::mutex> lk(s->mu);
-  rc = auto_batch(s, reqs, kappa_max, o, kappa, tier_out, st.data());
+  rc = auto_batch(s, std::move(reqs), kappa_max, o, kappa, tier_out, st.data());
   if (rc == 0) apply_status(b, o, st.data());
   return rc;
 }
@@ -1536,7 +1574,7 @@ int gbs_queue_evaluate_auto(gbs_session* s, int B, const int* funcs, const int* 
   for (int i = 0; i < B; ++i) reqs[i] = Req{funcs[i], kTierFp64, dims[i], mats + 2 * offsets[i]};
   std::vector<int> st(B);
   std::lock_guard<std::mutex> lk(s->mu);
-  const int rc = auto_batch(s, reqs, kappa_max, out, kappa, tier_out, st.data());
+  const int rc = auto_batch(s, std::move(reqs), kappa_max, out, kappa, tier_out, st.data());
   if (rc) return rc;
   if (status) std::memcpy(status, st.data(), sizeof(int) * B);
   apply_status(B, out, st.data());
@@ -1556,7 +1594,7 @@ int gbs_queue_evaluate_auto_ptrs(gbs_session* s, int B, const int* funcs, const 
   }
   std::vector<int> st(B);
   std::lock_guard<std::mutex> lk(s->mu);
-  const int rc = auto_batch(s, reqs, kappa_max, out, kappa, tier_out, st.data());
+  const int rc = auto_batch(s, std::move(reqs), kappa_max, out, kappa, tier_out, st.data());
   if (rc) return rc;
   if (status) std::memcpy(status, st.data(), sizeof(int) * B);
   apply_status(B, out, st.data());
@@ -1718,7 +1756,10 @@ namespace gbsb {
 static size_t req_bytes(const SrvReq& r) {
   const size_t d = (size_t)r.dim + 1;
   size_t items = 1;
-  if (r.fn == kFnHaf || r.fn == kFnLhaf) items = (size_t)1 << std::max(0, (int)(d / 2) - 7);
+  if (r.fn == kFnHaf || r.fn == kFnLhaf) {
+    items = (size_t)1 << std::max(0, (int)(d / 2) - kHafItemLog2);
+    if (r.tier == kTierKappa) items += (size_t)1 << std::max(0, (int)(d / 2) - kTermsItemLog2);  // terms
+  }
   return d * d * 16 + items * 48 + 256;
 }
 
@@ -1869,7 +1910,7 @@ int gbs_server_open(int n_slots, long long budget_bytes, int max_batch, gbs_serv
   // bytes of matrix and 48 bytes per work item), so serving never reallocates
   // (at most 256 MB of matrices per slot up front; a larger budget grows on demand)
   const size_t rbytes = std::min<size_t>(sv->budget, (size_t)256 << 20);
-  const size_t insts = std::min<size_t>((size_t)sv->max_batch, rbytes / 256 + 1);
+  const size_t insts = 2 * std::min<size_t>((size_t)sv->max_batch, rbytes / 256 + 1);  // auto: value and terms
   for (Slot& sl : sv->slots) {
     int rc = session_open(&sl.s);
     if (rc == 0) rc = session_reserve(sl.s, rbytes, rbytes / 48 + 1, insts);

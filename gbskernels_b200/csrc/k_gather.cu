@@ -43,7 +43,8 @@ cudaError_t launch_gather(const GatherDesc* descs, int n, const int* idx, double
 
 // Device-resident results: scatter of a plan's results from instance order (the
 // session's result arrays, grouped per launch) to request order in a caller-owned
-// device block, with no host round trip.  map[k] = destination index of instance k;
+// device block, with no host round trip.  map[k] = destination index i of instance k; ~(2 i) of
+// one that gives the aux alone (indicator terms), ~(2 i + 1) of one that gives all but the aux;
 // trivial requests (n = 0, odd hafnian) come as (index, re, im, aux).  A non-ok
 // status carries a NaN value (the work-item kernel already wrote it; the host
 // path applies the same convention).  Reference counterpart of the resident
@@ -68,8 +69,14 @@ __global__ void __launch_bounds__(256) scatter_kernel(ScatterArgs a) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < total; k += gridDim.x * blockDim.x) {
     int i, st;
     double re, im, x;
+    bool aux = a.write_aux != 0, value = true;
     if (k < a.ni) {
       i = a.map[k];
+      if (i < 0) {
+        value = (~i & 1) != 0;
+        aux = aux && !value;
+        i = ~i >> 1;
+      }
       st = a.st[k];
       re = a.out[2 * (size_t)k];
       im = a.out[2 * (size_t)k + 1];
@@ -83,9 +90,10 @@ __global__ void __launch_bounds__(256) scatter_kernel(ScatterArgs a) {
       im = a.tval[3 * t + 1];
       x = a.tval[3 * t + 2];
     }
+    if (aux) a.daux[i] = x;
+    if (!value) continue;
     a.dval[2 * (size_t)i] = re;
     a.dval[2 * (size_t)i + 1] = im;
-    if (a.write_aux) a.daux[i] = x;
     a.dst[i] = st;
   }
 }

@@ -3,6 +3,6 @@
 #include "gbs_items.cuh"
 
 namespace gbsb {
-#define GBSB_LIST_HAF(X) X(br1(kFnHaf, kTierFp64)) X(br1(kFnHaf, kTierKappa)) X(br1(kFnLhaf, kTierFp64)) X(br1(kFnLhaf, kTierKappa)) X(kBrHafLhafFp64)
+#define GBSB_LIST_HAF(X) X(br1(kFnHaf, kTierFp64)) X(br1(kFnHaf, kTierKappa)) X(br1(kFnLhaf, kTierFp64)) X(br1(kFnLhaf, kTierKappa)) X(kBrTermsLarge) X(kBrHafLhafFp64)
 GBSB_DEFINE_GROUP(haf, GBSB_LIST_HAF)
 }  // namespace gbsb
