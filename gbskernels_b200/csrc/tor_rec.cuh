@@ -203,12 +203,11 @@ __host__ __device__ inline TorRecState tor_rec_walked(const TorRecLayout& R, con
   return TorRecState{tor_rec_dfs(R, R.mW + s), R.f - (R.mW + s)};
 }
 
-// The entry of O read for row i, column j <= i of M.  O is meant to be symmetric; of one that
-// is not, the torontonian reads the lower triangle in the order (mode, x before p), as the
-// reference does, but for the block of the last `tail` modes (5, double-double 4) against the
-// modes before them, where it reads the upper one.
-__host__ __device__ inline void tor_rec_source(int k, int tail, int i, int j, int& row, int& col) {
-  const int mi = k - 1 - (i >> 1), mj = k - 1 - (j >> 1);  // modes, mi <= mj
+// The entry of O read for row i, column j <= i of M, which belong to the modes mi <= mj.  O is
+// meant to be symmetric; of one that is not, the torontonian reads the lower triangle in the
+// order (mode, x before p), as the reference does, but for the block of the last `tail`
+// modes (5, double-double 4) against the modes before them, where it reads the upper one.
+__host__ __device__ inline void tor_rec_source(int k, int tail, int i, int mi, int j, int mj, int& row, int& col) {
   const int a = mi + (i & 1) * k, b = mj + (j & 1) * k;
   const bool upper = mi == mj || (mi < k - tail && mj >= k - tail);
   row = upper ? a : b;
@@ -446,19 +445,25 @@ static __device__ __noinline__ bool tor_rec_item(const double* __restrict__ Oc, 
   constexpr int TAIL = TorRec<S>::kTail;
   const S z{};
   const int dim = 2 * k;
-  for (int e = lane; e < tor_rec_entries(k); e += 32) {
-    const int i = tor_rec_row(e), j = e - i * (i + 1) / 2;
+  // the modes that the pattern leaves out are not staged at all: their rows lie behind those
+  // of every later step (20 modes in 2^14 items of 2^6 subsets: 0.75 ms, 0.79 with them)
+  const uint32_t inc = pat & (g < 32 ? (1u << g) - 1u : 0xffffffffu);
+  const int inc0 = __popc(inc), ks = R.f + inc0;
+  int* modes = reinterpret_cast<int*>(ws + R.noff * TorRec<S>::W);  // included modes, the last first
+  if ((inc >> lane) & 1u) modes[inc0 - 1 - __popc(inc & ((1u << lane) - 1u))] = lane;
+  __syncwarp();
+  for (int e = lane; e < tor_rec_entries(ks); e += 32) {
+    const int i = tor_rec_row(e), j = e - i * (i + 1) / 2, si = i >> 1, sj = j >> 1;
     int r, c;
-    tor_rec_source(k, TorRec<S>::kOrder, i, j, r, c);
+    tor_rec_source(k, TorRec<S>::kOrder, i, si < R.f ? k - 1 - si : modes[si - R.f], j,
+                   sj < R.f ? k - 1 - sj : modes[sj - R.f], r, c);
     ts_st(ws, e, ts_m(Oc, dim, r, c, z));
   }
   if (lane == 0) ts_st(ws, R.t, ts_make(1.0, z));
   __syncwarp();
   bool ok = true;
   const TorRecState root{0, 0};
-  for (int j = 0; j < g; ++j)
-    if ((pat >> j) & 1u) tor_rec_include<S>(ws, R, k - j, 1, [&](int) { return root; }, 0, 0, lane, ok);
-  const int inc0 = __popc(pat & (g < 32 ? (1u << g) - 1u : 0xffffffffu));
+  for (int m = ks; m > R.f; --m) tor_rec_include<S>(ws, R, m, 1, [&](int) { return root; }, 0, 0, lane, ok);
   S sum = ts_make(0.0, z);
   double acc = 0.0;
   const uint32_t nT = 1u << (R.f - R.mW);
@@ -480,18 +485,18 @@ static __device__ __noinline__ bool tor_rec_item(const double* __restrict__ Oc, 
     }
     if (lane < (1 << (R.mW - R.mt))) {
       const TorRecState s = tor_rec_node(R, w, R.mt, lane);
-      const int inc = inc0 + __popc(Tm) + __popc(lane);
+      const int in = inc0 + __popc(Tm) + __popc(lane);
       const S t = ts_ld(ws, R.t + s.t, z);
       TorRecSum<S, AUX> f;
       switch (R.mt) {
-        case 0: f = tor_rec_tail_load<S, AUX, 0>(ws, s.off, t, 2 * inc, rho, ok); break;
-        case 1: f = tor_rec_tail_load<S, AUX, 1>(ws, s.off, t, 2 * inc, rho, ok); break;
-        case 2: f = tor_rec_tail_load<S, AUX, 2>(ws, s.off, t, 2 * inc, rho, ok); break;
+        case 0: f = tor_rec_tail_load<S, AUX, 0>(ws, s.off, t, 2 * in, rho, ok); break;
+        case 1: f = tor_rec_tail_load<S, AUX, 1>(ws, s.off, t, 2 * in, rho, ok); break;
+        case 2: f = tor_rec_tail_load<S, AUX, 2>(ws, s.off, t, 2 * in, rho, ok); break;
         default:
-          if (TAIL == 3 || R.mt == 3) f = tor_rec_tail_load<S, AUX, 3>(ws, s.off, t, 2 * inc, rho, ok);
-          else f = tor_rec_tail_load<S, AUX, TAIL>(ws, s.off, t, 2 * inc, rho, ok);
+          if (TAIL == 3 || R.mt == 3) f = tor_rec_tail_load<S, AUX, 3>(ws, s.off, t, 2 * in, rho, ok);
+          else f = tor_rec_tail_load<S, AUX, TAIL>(ws, s.off, t, 2 * in, rho, ok);
       }
-      sum = ts_add(sum, ((k - R.mt - inc) & 1) ? ts_neg(f.v) : f.v);
+      sum = ts_add(sum, ((k - R.mt - in) & 1) ? ts_neg(f.v) : f.v);
       if (AUX == 1) acc += f.a;
       if (AUX == 2) acc = ru_add(ru_add(acc, f.a), ts_sum_err(sum));
     }

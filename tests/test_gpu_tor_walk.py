@@ -155,3 +155,35 @@ def test_splits_with_more_free_modes_than_one_walk_takes(gpu, lib, orc, n):
         # the double-double sum's own error, kappa 2^-104 or so, is below its rounding
         assert (np.abs(dd - dd0) <= (2.0 ** -52 + 1e-28 * kappa) * np.abs(dd0)).all(), split
         assert np.array([d["cancellation"] for d in dk]) == pytest.approx(kappa, rel=1e-6), split
+
+
+def test_one_proof_serves_the_items_of_its_instance_only(gpu):
+    # certified torontonians of several items each, among instances of other tiers and some
+    # whose proof fails: values, bounds and refusals are those of each one alone
+    mats, tiers = [], []
+    for i in range(24):
+        n = (15, 9, 16, 17)[i % 4]
+        O = phys_O(n, 1.0 + i % 3)
+        if i % 7 == 3:
+            w, V = np.linalg.eigh(np.eye(2 * n) - O)
+            w[0] = -0.05
+            O = np.eye(2 * n) - (V * w) @ V.T
+            O = (O + O.T) / 2
+        mats.append(O.astype(complex))
+        tiers.append(("certified", "certified", "certified-dd", "fp64", "certified")[i % 5])
+    with gpu.Workspace() as ws:
+        out, aux, st = ws.evaluate_full(["tor"] * 24, mats, tiers)
+        for i in range(24):
+            o, a, s = ws.evaluate_full(["tor"], [mats[i]], [tiers[i]])
+            assert np.array_equal(o[0], out[i], equal_nan=True) and a[0] == aux[i] and s[0] == st[i], (i, tiers[i])
+    assert st.any() and not st.all()
+
+
+@pytest.mark.parametrize("n", [10, 16, 18])
+def test_single_large_splits_agree(gpu, n):
+    O = phys_O(n)
+    dd, ddd = gpu.tor_single(O, dd=True)
+    for groups in (None, 0, 5, 9, min(n, 14), n):
+        v, d = gpu.tor_single(O, groups=groups, certified=True)
+        assert v == gpu.tor_single(O, groups=groups), groups
+        assert abs(v - dd) <= d["abs_error_bound"] + ddd["abs_error_bound"], groups

@@ -102,17 +102,21 @@ extern "C" int t_tor_rec_item(const double* O, int k, int g, unsigned lo, int is
     const unsigned pat = tor_rec_pattern(lo, p, g, g2);
     x.w.assign(R.rho, 0.0);
     x.set.assign(R.rho, 0);
-    for (int e = 0; e < tor_rec_entries(k); ++e) {
+    const int inc0 = __builtin_popcount(pat), ks = f + inc0;
+    std::vector<int> modes;  // included ones of the first g2, the last first
+    for (int j = g2 - 1; j >= 0; --j)
+      if ((pat >> j) & 1u) modes.push_back(j);
+    if (inc0 > 2 * (1 << kTorRecWide) / 2 || R.noff + (1 << kTorRecWide) / 2 > R.rho) ++x.bad;  // the list's place
+    auto mode = [&](int r) { return r / 2 < f ? k - 1 - r / 2 : modes[r / 2 - f]; };
+    for (int e = 0; e < tor_rec_entries(ks); ++e) {
       const int i = tor_rec_row(e), j = e - i * (i + 1) / 2;
       int a, b;
-      tor_rec_source(k, is_dd ? TorRec<dd>::kOrder : TorRec<double>::kOrder, i, j, a, b);
+      tor_rec_source(k, is_dd ? TorRec<dd>::kOrder : TorRec<double>::kOrder, i, mode(i), j, mode(j), a, b);
       x.put(e, (a == b ? 1.0 : 0.0) - O[a * dim + b]);
     }
     x.put(R.t, 1.0);
     const TorRecState root{0, 0};
-    for (int j = 0; j < g2; ++j)
-      if ((pat >> j) & 1u) x.include(k - j, 1, [&](int) { return root; }, 0, 0);
-    const int inc0 = __builtin_popcount(pat);
+    for (int m = ks; m > f; --m) x.include(m, 1, [&](int) { return root; }, 0, 0);
     for (unsigned Tm = 0; Tm < (1u << (R.f - R.mW)); ++Tm) {
       if (Tm) {
         const int s = __builtin_ctz(Tm), m = R.mW + 1 + s;
