@@ -150,7 +150,8 @@ __device__ __forceinline__ void hz_st(int i, double v) { smem[i] = v; }
 __device__ __forceinline__ void hz_st(int i, const ddc& v) { st_ddc(smem + 4 * i, v); }
 __device__ __forceinline__ void hz_st(int i, cplx v) { reinterpret_cast<double2*>(smem)[i] = make_double2(v.re, v.im); }
 
-// Loads by shared-memory byte address (an address select per load, no branch).
+// Loads by shared-memory byte address (an address select per load, no branch).  The compiler
+// does not see that they read what hz_st wrote: haf_rec_op keeps its stores behind them.
 __device__ __forceinline__ uint32_t hz_addr(int i, int bytes) {
   return (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)(i * bytes);
 }
@@ -182,6 +183,7 @@ struct HafRecLane {
 template <int T, typename Z>
 __device__ __noinline__ void haf_rec_op(HafRecLane L, double bias) {
   constexpr int B = (int)sizeof(Z);
+  asm volatile("" ::: "memory");  // stores before the step stay before its loads
   const uint32_t zero = hz_addr(L.zero, B);
   const uint32_t str = (uint32_t)(L.str * B);
   Z acc[T + 2];
@@ -208,6 +210,7 @@ __device__ __noinline__ void haf_rec_op(HafRecLane L, double bias) {
     bstr = str;
     L.lim = L.limb = L.lim2;
   }
+  asm volatile("" ::: "memory");  // a step in place overwrites words that it has read
   if (L.dst >= 0) {
 #pragma unroll
     for (int c = 0; c < T + 2; ++c) hz_st(L.dst + c * L.dstr, acc[c]);
