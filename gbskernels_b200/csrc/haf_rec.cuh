@@ -31,7 +31,8 @@
 //     suffice.  T is a template parameter: a rolled loop (Horner's rule, P <- z P + a v)
 //     spent as many register moves as FMAs on the shift
 //     (measured, complex 28 x 28, 256 instances: 19 us each, 33 us rolled, 47 us with a
-//     branch instead of an address select around every load; 250 us by power traces);
+//     branch instead of an address select around every load; 250 us by power traces; 16 us
+//     since e is kept where g' goes, which makes room for another warp);
 //   * coefficient-major planes [c][pair] with pair index j(j-1)/2 + k, the pair taken
 //     next being the two highest vertices: leaving a pair out is a view (shorter
 //     planes), the operands of a lane are rows of the two taken vertices (contiguous

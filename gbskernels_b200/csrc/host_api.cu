@@ -645,7 +645,8 @@ static int plan_build(gbs_session* s, const std::vector<Req>& reqs, const RunOpt
   if (e != cudaSuccess) return fail(e, "synchronising the session stream");
   // ---- pack matrices (odd loop hafnians augmented by A (+) [1]) and upload once: with the
   // queues when that is small and nothing on the device has to read it before, else while
-  // the queues are still being written
+  // the queues are still being written (eight complex 8 x 8 hafnians: 48.5 us a call in one
+  // upload, 52 in two; 64 of them 64.5 and 70; from 256 KB on the same within the noise)
   bool one_upload = mat_bytes + meta_bytes <= (256u << 10);
   for (int i = 0; i < B && one_upload; ++i) one_upload = !reqs[i].state;
   // a large batch of real matrices travels as it is and is widened on the device

@@ -24,7 +24,7 @@
 //   * five modes breadth-first: up to 32 nodes, lanes over (node, entry);
 //   * the last kTail modes (4; double-double 3) per lane in registers: lane = node, the
 //     2^kTail subsets by a compile-time recursion, the last mode by its 2 x 2 determinant.
-// Bound by latency and the issue of its instruction stream (about 3,700 warp instructions
+// Bound by latency and the issue of its instruction stream (about 3,200 warp instructions
 // per 512 subsets, a quarter of them FP64), not by the FP64 pipe.  Measured, against one
 // 10 x 10 factorisation per lane and subset: 64 x 20 modes 5.98 -> 1.43 ms, 512 x 12 modes
 // 0.340 -> 0.091 ms.
