@@ -445,19 +445,28 @@ static __device__ __noinline__ bool tor_rec_item(const double* __restrict__ Oc, 
   constexpr int TAIL = TorRec<S>::kTail;
   const S z{};
   const int dim = 2 * k;
-  // the modes that the pattern leaves out are not staged at all: their rows lie behind those
-  // of every later step (20 modes in 2^14 items of 2^6 subsets: 0.75 ms, 0.79 with them)
   const uint32_t inc = pat & (g < 32 ? (1u << g) - 1u : 0xffffffffu);
   const int inc0 = __popc(inc), ks = R.f + inc0;
-  int* modes = reinterpret_cast<int*>(ws + R.noff * TorRec<S>::W);  // included modes, the last first
-  if ((inc >> lane) & 1u) modes[inc0 - 1 - __popc(inc & ((1u << lane) - 1u))] = lane;
-  __syncwarp();
-  for (int e = lane; e < tor_rec_entries(ks); e += 32) {
-    const int i = tor_rec_row(e), j = e - i * (i + 1) / 2, si = i >> 1, sj = j >> 1;
-    int r, c;
-    tor_rec_source(k, TorRec<S>::kOrder, i, si < R.f ? k - 1 - si : modes[si - R.f], j,
-                   sj < R.f ? k - 1 - sj : modes[sj - R.f], r, c);
-    ts_st(ws, e, ts_m(Oc, dim, r, c, z));
+  if (g == 0) {
+    for (int e = lane; e < tor_rec_entries(k); e += 32) {
+      const int i = tor_rec_row(e), j = e - i * (i + 1) / 2;
+      int r, c;
+      tor_rec_source(k, TorRec<S>::kOrder, i, k - 1 - (i >> 1), j, k - 1 - (j >> 1), r, c);
+      ts_st(ws, e, ts_m(Oc, dim, r, c, z));
+    }
+  } else {
+    // the modes that the pattern leaves out are not staged at all: their rows lie behind those
+    // of every later step (20 modes in 2^14 items of 2^6 subsets: 0.75 ms, 0.79 with them)
+    int* modes = reinterpret_cast<int*>(ws + R.noff * TorRec<S>::W);  // included modes, the last first
+    if ((inc >> lane) & 1u) modes[inc0 - 1 - __popc(inc & ((1u << lane) - 1u))] = lane;
+    __syncwarp();
+    for (int e = lane; e < tor_rec_entries(ks); e += 32) {
+      const int i = tor_rec_row(e), j = e - i * (i + 1) / 2, si = i >> 1, sj = j >> 1;
+      int r, c;
+      tor_rec_source(k, TorRec<S>::kOrder, i, si < R.f ? k - 1 - si : modes[si - R.f], j,
+                     sj < R.f ? k - 1 - sj : modes[sj - R.f], r, c);
+      ts_st(ws, e, ts_m(Oc, dim, r, c, z));
+    }
   }
   if (lane == 0) ts_st(ws, R.t, ts_make(1.0, z));
   __syncwarp();
